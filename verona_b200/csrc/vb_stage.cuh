@@ -493,12 +493,11 @@ cudaError_t dispatch_stage_dim(int rec, int rs, const StageParams& p, const Stag
     return cudaErrorInvalidValue;
 }
 
-template <typename R> inline bool zm_fits(const StageParams& p);
 template <typename R>
 cudaError_t dispatch_stage_zm(int rec, int rs, const StageParams& p, const StageBufs<R>& b, cudaStream_t s);
 
-// 3D grids whose x/y interior extents are multiples of the z-marching tile
-// use k_stage_zm; everything else (1D, 2D, ragged 3D) the box-tile k_stage.
+// 3D grids use the z-marching kernels (unless force_box); 1D and 2D the
+// box-tile k_stage.
 // *kernels receives the number of kernels launched (2 for a split z-march
 // stage, whose con2prim runs in k_c2p; else 1).
 template <typename R>
@@ -517,7 +516,7 @@ cudaError_t launch_stage(int dims, int rec, int rs, const StageParams& p, const 
         return launch_c2p<R>(p, b, s);
     }
     if (dims == 3) {
-        if (zm_fits<R>(p) && !p.force_box) {
+        if (!p.force_box) {
             *kernels = p.split && !p.skip_c2p ? 2 : 1;
             return dispatch_stage_zm<R>(rec, rs, p, b, s);
         }

@@ -3,8 +3,9 @@
 // Same arithmetic, per cell, as the box-tile k_stage and as the reference
 // (src/3dim/algos.jl:14-200 + src/3dim/structs.jl:218-628), organised for the
 // hardware:
-//   * a CTA owns TX x TY columns and walks one z-range of LZ cells; each
-//     thread owns one (x, y) column;
+//   * a CTA owns TX x TY columns and walks one z-range of lz cells (z_range);
+//     each thread owns one (x, y) column; on the last tile of a ragged extent
+//     the threads past the interior run on clamped columns and store nothing;
 //   * the z-stencil of a column (planes k-1 .. k+3, all five variables)
 //     lives in registers and slides up one plane per step, so every z-face
 //     is reconstructed once and the z-halo is read once per range;
@@ -20,6 +21,8 @@
 // the floors, as in k_stage.
 #pragma once
 #include "vb_ns.h"
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "vb_stage.cuh"
@@ -74,8 +77,8 @@ __device__ __forceinline__ void recon_floored(const R* q, int s, R fl, int v, R&
     }
 }
 
-template <int REC, int RS, typename R, int TX, int TY, int LZ, int MINB, bool SPLIT>
-__global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, StageBufs<R> b) {
+template <int REC, int RS, typename R, int TX, int TY, int MINB, bool SPLIT>
+__global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, StageBufs<R> b, int lz) {
     using G = ZmGeom<TX, TY>;
     constexpr int NV = 5, NT = G::NT, EX = G::EX, PLN = G::PLN, FN = G::FN, QXN = G::QXN;
     constexpr int FXR = TX + 1;  // x faces per row
@@ -91,9 +94,13 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
     const int tid = threadIdx.x;
     const int tx = tid % TX, ty = tid / TX;
     const int i0 = NG + blockIdx.x * TX, j0 = NG + blockIdx.y * TY;
-    const int i = i0 + tx, j = j0 + ty;
-    const int z0 = NG + blockIdx.z * LZ;
-    const int zend = min(z0 + LZ, p.n[2] - NG);
+    // ragged tiles: columns past the padded extents read the last padded column;
+    // only interior columns (mine) touch U and the output
+    const int ilast = p.n[0] - 1, jlast = p.n[1] - 1;
+    const int i = min(i0 + tx, ilast), j = min(j0 + ty, jlast);
+    const bool mine = i0 + tx < p.n[0] - NG && j0 + ty < p.n[1] - NG;
+    const int z0 = NG + blockIdx.z * lz;
+    const int zend = min(z0 + lz, p.n[2] - NG);
     const long long sy = p.sy, sz = p.sz, vs = p.vs;
     const long long col = i + sy * j;
     const R fl = R(p.floor_);
@@ -135,7 +142,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
     for (int k = z0; k < zend; ++k) {
         const long long c = col + sz * k;
         DivAcc<R> acc;
-        acc.init(b.Us, vs, c);
+        if (mine) acc.init(b.Us, vs, c);
 
         // stage plane k: own value, then the x-halo (6 per row) and y-halo (6 per column)
         __syncthreads();
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
                 hx = e2 % TX;
                 hy = s6 < 3 ? s6 - 3 : TY + s6 - 3;
             }
-            const long long gc = (i0 + hx) + sy * (j0 + hy) + sz * k;
+            const long long gc = min(i0 + hx, ilast) + sy * min(j0 + hy, jlast) + sz * k;
 #pragma unroll
             for (int v = 0; v < NV; ++v) sPl[v * PLN + (hy + 3) * EX + hx + 3] = b.Pin[v * vs + gc];
         }
@@ -278,7 +285,9 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
 
         // RK combination, con2prim (guess = plane k of this stage's P), Limit;
         // in split mode only U is written here and k_c2p finishes the cell
-        if (SPLIT) {
+        if (!mine) {
+            // nothing to store
+        } else if (SPLIT) {
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 double u = acc.result(v, b.Us, vs, c);
@@ -329,12 +338,46 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
 
 // Tile shape of the z-marching kernel per bulk type.
 template <typename R> struct ZmCfg;
-template <> struct ZmCfg<float> { static constexpr int TX = 32, TY = 8, LZ = 64, MINB = 3, MINB_SPLIT = 4; };
-template <> struct ZmCfg<double> { static constexpr int TX = 32, TY = 8, LZ = 64, MINB = 2, MINB_SPLIT = 2; };
+template <> struct ZmCfg<float> { static constexpr int TX = 32, TY = 8, MINB = 3, MINB_SPLIT = 4; };
+template <> struct ZmCfg<double> { static constexpr int TX = 32, TY = 8, MINB = 2, MINB_SPLIT = 2; };
 
-template <typename R> inline bool zm_fits(const StageParams& p) {
-    using C = ZmCfg<R>;
-    return (p.n[0] - 2 * NG) % C::TX == 0 && (p.n[1] - 2 * NG) % C::TY == 0 && p.n[2] - 2 * NG >= 1;
+// Planes per z range of a z-marching kernel. A range costs its planes plus a
+// prologue (the window's loads, two reconstructions and one flux: 0.6 planes),
+// and CTAs run on `slots` places: x = CTAs / slots rounds of them take between
+// x + 1/2 (they drift apart) and ceil(x) times a range's cost; the length, in
+// steps of `step` planes and at most Z_RANGE_MAX, minimises the mean of the
+// two to 1 %, the longer of those. Measured on the z-pair kernel at 320 x 128 x 128
+// (160 columns, 296 slots): ranges of 64 planes 0.482 ms, 32 0.392, 16 0.355,
+// 12 (chosen) 0.348, 8 0.364, 4 0.378; at 512^3 64 (chosen) 8.17, 32 8.19,
+// 16 8.33, 128 8.19, 512 8.36 ms. On a 64 x 48 x 48 FP64 grid a fixed 64 ran 12
+// CTAs of 48 planes: 1008 us a stage, against 85 us.
+constexpr int Z_RANGE_MAX = 64;
+inline int z_range(long long columns, int nz, int slots, int step) {
+    int best = 0;
+    double cost = 0.0;
+    // gridDim.z is at most 65535
+    for (int lz = (std::max(step, (nz + 65534) / 65535) + step - 1) / step * step;; lz += step) {
+        const double x = (double)(columns * ((nz + lz - 1) / lz)) / slots;
+        const double c = (x <= 1.0 ? 1.0 : 0.5 * (std::ceil(x) + x + 0.5)) * (std::min(lz, nz) + 0.6);
+        if (!best || c <= 1.01 * cost) best = lz;
+        if (cost == 0.0 || c < cost) cost = c;
+        if (lz >= nz || lz >= Z_RANGE_MAX) return best;
+    }
+}
+inline int sm_count() {
+    static int cached[64] = {0};  // per device; racing writers store the same value
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = cached[dev & 63];
+    if (!n && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return n;
+}
+// grid of a z-marching kernel with TX x TY column tiles; *lz: its planes per range
+inline dim3 z_march_grid(const StageParams& p, int TX, int TY, int ctas_per_sm, int step, int* lz) {
+    const int nx = p.n[0] - 2 * NG, ny = p.n[1] - 2 * NG, nz = p.n[2] - 2 * NG;
+    const int tx = (nx + TX - 1) / TX, ty = (ny + TY - 1) / TY;
+    *lz = z_range((long long)tx * ty, nz, ctas_per_sm * sm_count(), step);
+    return dim3(tx, ty, (nz + *lz - 1) / *lz);
 }
 
 // Split-mode con2prim: one thread per interior cell, no barriers, no shared
@@ -480,7 +523,8 @@ template <int REC, int RS, typename R, bool SPLIT>
 cudaError_t launch_stage_zm_t(const StageParams& p, const StageBufs<R>& b, cudaStream_t s) {
     using C = ZmCfg<R>;
     using G = ZmGeom<C::TX, C::TY>;
-    auto kern = k_stage_zm<REC, RS, R, C::TX, C::TY, C::LZ, SPLIT ? C::MINB_SPLIT : C::MINB, SPLIT>;
+    constexpr int MINB = SPLIT ? C::MINB_SPLIT : C::MINB;
+    auto kern = k_stage_zm<REC, RS, R, C::TX, C::TY, MINB, SPLIT>;
     const size_t smem = G::template smem_bytes<R>();
     static unsigned long long attr_set = 0;
     int dev = 0;
@@ -492,8 +536,9 @@ cudaError_t launch_stage_zm_t(const StageParams& p, const StageBufs<R>& b, cudaS
         if (e != cudaSuccess) return e;
         attr_set |= 1ULL << (dev & 63);
     }
-    dim3 grid((p.n[0] - 2 * NG) / C::TX, (p.n[1] - 2 * NG) / C::TY, (p.n[2] - 2 * NG + C::LZ - 1) / C::LZ);
-    kern<<<grid, C::TX * C::TY, smem, s>>>(p, b);
+    int lz;
+    const dim3 grid = z_march_grid(p, C::TX, C::TY, MINB, 1, &lz);
+    kern<<<grid, C::TX * C::TY, smem, s>>>(p, b, lz);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !SPLIT || p.skip_c2p) return e;
     const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG) * (p.n[2] - 2 * NG);
@@ -512,7 +557,7 @@ cudaError_t launch_stage_zm(const StageParams& p, const StageBufs<R>& b, cudaStr
 }
 
 template <typename R> int stage_div_in_pout(int dims, int rec, int rs, const StageParams& p) {
-    if (!std::is_same<R, float>::value || dims != 3 || p.force_box || !zm_fits<R>(p)) return 0;
+    if (!std::is_same<R, float>::value || dims != 3 || p.force_box) return 0;
     return p.pairs && zp_available(rec, rs) && p.skip_c2p && p.want_div ? 1 : 0;
 }
 
@@ -522,7 +567,7 @@ template <typename R> int stage_div_in_pout(int dims, int rec, int rs, const Sta
 // by launch_c2p
 template <typename R> int stage_split_c2p(int dims, const StageParams& p) {
     if (dims == 2) return p.split && !p.skip_c2p ? 1 : 0;
-    return dims == 3 && !p.force_box && zm_fits<R>(p) && p.split && !p.skip_c2p ? 1 : 0;
+    return dims == 3 && !p.force_box && p.split && !p.skip_c2p ? 1 : 0;
 }
 
 template <typename R>
