@@ -35,7 +35,7 @@ VB_HD void solve3(const double* A, const double* b, double* x) {
 
 // 1D UtoP, src/1dim/structs.jl:78-105 (F_ptoU :48-54, Jacobian :32-46).
 // The stop rule drops the last delta. Returns the iteration count.
-VB_HD int c2p_1d(double g, int n_iter, double tol, const double* U, double* P) {
+VB_HD int c2p_1d_general(double g, int n_iter, double tol, const double* U, double* P) {
     double x1 = P[0], x2 = P[1], x3 = P[2];
     int it;
     for (it = 1; it <= n_iter; ++it) {
@@ -69,6 +69,69 @@ VB_HD int c2p_1d(double g, int n_iter, double tol, const double* U, double* P) {
     P[1] = x2;
     P[2] = x3;
     return it;
+}
+
+// ---- con2prim on the branch-free divide and square root (vb_fp64.cuh) ----------
+// The same Newton iterations as the general forms, operation for operation;
+// every divisor and dividend is tested where it arises, and a cell that leaves
+// the range (or whose iterates do) is solved by the general form from its guess.
+constexpr int C2P_DECLINED = -1000000;  // no result code reaches it: n_iter is at most 100000
+
+// moderate or zero, as a dividend or a factor
+VB_HD bool c2p_moderate(double x) { return d64::zero_or_in<-300, 100>(x); }
+
+VB_HD int c2p_1d_fast(double g, int n_iter, double tol, const double* U, double* P) {
+    double x1 = P[0], x2 = P[1], x3 = P[2];
+    int it;
+    for (it = 1; it <= n_iter; ++it) {
+        const double gam = d64::root(sq(x3) + 1.0);
+        const double w = g * x2 + x1;
+        const double f0 = gam * x1 - U[0];
+        const double f1 = (g - 1.0) * x2 - sq(gam) * w - U[1];
+        const double f2 = x3 * gam * w - U[2];
+        const d64::Div ig = d64::divisor(gam);
+        const double J0 = gam;
+        const double J6 = d64::quot_s(x1 * x3, ig);
+        const double J1 = -sq(gam);
+        const double J4 = (g - 1.0) - sq(gam) * g;
+        const double J7 = -2.0 * x3 * w;
+        const double J2 = gam * x3;
+        const double J5 = gam * x3 * g;
+        const double J8 = d64::quot((2.0 * sq(x3) + 1.0), ig) * w;
+        // solve3 with A = [J0 0 J6; J1 J4 J7; J2 J5 J8]
+        const double c1 = J4 * J8 - J5 * J7;
+        const double c2 = J5 * J6 - 0.0 * J8;
+        const double c3 = 0.0 * J7 - J4 * J6;
+        const double det = J0 * c1 + J1 * c2 + J2 * c3;
+        const d64::Div id = d64::divisor(det);
+        const double n0 = (J4 * J8 - J7 * J5) * f0 + (J6 * J5 - 0.0 * J8) * f1 + (0.0 * J7 - J6 * J4) * f2;
+        const double n1 = (J7 * J2 - J1 * J8) * f0 + (J0 * J8 - J6 * J2) * f1 + (J6 * J1 - J0 * J7) * f2;
+        const double n2 = (J1 * J5 - J4 * J2) * f0 + (0.0 * J2 - J0 * J5) * f1 + (J0 * J4 - 0.0 * J1) * f2;
+        const double d0 = d64::quot_s(n0, id), d1 = d64::quot_s(n1, id), d2 = d64::quot_s(n2, id);
+        const double s = sq(d0) + sq(d1) + sq(d2);
+        const double norm = d64::is_zero(s) ? s : d64::root(s);
+        if (!(c2p_moderate(x1) && c2p_moderate(x2) && c2p_moderate(x3) && d64::abs_in<-300, 300>(det) &&
+              d64::zero_or_in<-600, 600>(n0) && d64::zero_or_in<-600, 600>(n1) && d64::zero_or_in<-600, 600>(n2) &&
+              d64::zero_or_in<-900, 900>(s)))
+            return C2P_DECLINED;
+        if (norm < tol) break;
+        x1 = x1 - d0;
+        x2 = x2 - d1;
+        x3 = x3 - d2;
+    }
+    P[0] = x1;
+    P[1] = x2;
+    P[2] = x3;
+    return it;
+}
+
+VB_HD int c2p_1d(double g, int n_iter, double tol, const double* U, double* P) {
+    const int r = c2p_1d_fast(g, n_iter, tol, U, P);
+    return r != C2P_DECLINED ? r : c2p_1d_general(g, n_iter, tol, U, P);
+}
+
+static __host__ __device__ VB_NOINLINE int c2p_1d_call(double g, int n_iter, double tol, const double* U, double* P) {
+    return c2p_1d(g, n_iter, tol, U, P);
 }
 
 // LU_dec_pivot!, src/2dim/structs.jl:121-208. Returns false on a row-wise
@@ -143,7 +206,7 @@ VB_HD bool lu_pivot4(double* A, double* t, double* x) {
 
 // 2D function_UtoP, src/2dim/structs.jl:249-330. Returns the iteration count,
 // -1 on a singular Jacobian.
-VB_HD int c2p_2d(double g, int n_iter, double tol, const double* U, double* P) {
+VB_HD int c2p_2d_general(double g, int n_iter, double tol, const double* U, double* P) {
     int it;
     for (it = 1; it <= n_iter; ++it) {
         double gam = sqrt(sq(P[2]) + sq(P[3]) + 1.0);
@@ -177,6 +240,131 @@ VB_HD int c2p_2d(double g, int n_iter, double tol, const double* U, double* P) {
         P[3] = P[3] - o[3];
     }
     return it;
+}
+
+// lu_pivot4 on the branch-free divide, each pivot's reciprocal formed once;
+// false in *ok where an operand leaves its range
+VB_HD bool lu_pivot4_fast(double* A, double* t, double* x, bool* ok) {
+#define I4(i, j) (((j)-1) * 4 + (i)-1)
+    double rn[4];
+#pragma unroll
+    for (int i = 1; i <= 4; ++i) {
+        double am = 0.0;
+#pragma unroll
+        for (int j = 1; j <= 4; ++j) {
+            const double tmp = fabs(A[I4(i, j)]);
+            if (tmp > am) am = tmp;
+        }
+        if (am == 0.0) return false;
+        *ok = *ok && d64::pos_in<-300, 300>(am);
+        rn[i - 1] = d64::quot(1.0, d64::divisor(am));
+    }
+    d64::Div piv_inv[4];
+#pragma unroll
+    for (int k = 1; k <= 4; ++k) {
+        int piv = k;
+        double pv = fabs(A[I4(k, k)]) * rn[k - 1];
+#pragma unroll
+        for (int i = k + 1; i <= 4; ++i) {
+            const double tmp = fabs(A[I4(i, k)]) * rn[i - 1];
+            if (tmp > pv) {
+                pv = tmp;
+                piv = i;
+            }
+        }
+#pragma unroll
+        for (int i = k + 1; i <= 4; ++i) {
+            const bool sw = piv == i;
+#pragma unroll
+            for (int j = 1; j <= 4; ++j) {
+                const double tmp = A[I4(k, j)];
+                A[I4(k, j)] = sw ? A[I4(i, j)] : tmp;
+                A[I4(i, j)] = sw ? tmp : A[I4(i, j)];
+            }
+            double tmp = t[k - 1];
+            t[k - 1] = sw ? t[i - 1] : tmp;
+            t[i - 1] = sw ? tmp : t[i - 1];
+            tmp = rn[k - 1];
+            rn[k - 1] = sw ? rn[i - 1] : tmp;
+            rn[i - 1] = sw ? tmp : rn[i - 1];
+        }
+        *ok = *ok && d64::abs_in<-300, 300>(A[I4(k, k)]);
+        piv_inv[k - 1] = d64::divisor(A[I4(k, k)]);
+#pragma unroll
+        for (int i = k + 1; i <= 4; ++i) {
+            *ok = *ok && d64::zero_or_in<-600, 600>(A[I4(i, k)]);
+            A[I4(i, k)] = d64::quot_s(A[I4(i, k)], piv_inv[k - 1]);
+#pragma unroll
+            for (int j = k + 1; j <= 4; ++j) A[I4(i, j)] = fma(-A[I4(i, k)], A[I4(k, j)], A[I4(i, j)]);
+        }
+    }
+#pragma unroll
+    for (int i = 1; i <= 4; ++i) {
+        x[i - 1] = t[i - 1];
+#pragma unroll
+        for (int j = 1; j <= i - 1; ++j) x[i - 1] = fma(-A[I4(i, j)], x[j - 1], x[i - 1]);
+    }
+#pragma unroll
+    for (int i = 4; i >= 1; --i) {
+#pragma unroll
+        for (int j = i + 1; j <= 4; ++j) x[i - 1] = fma(-A[I4(i, j)], x[j - 1], x[i - 1]);
+        *ok = *ok && d64::zero_or_in<-600, 600>(x[i - 1]);
+        x[i - 1] = d64::quot_s(x[i - 1], piv_inv[i - 1]);
+    }
+#undef I4
+    return true;
+}
+
+VB_HD int c2p_2d_fast(double g, int n_iter, double tol, const double* U, double* Pio) {
+    double P[4] = {Pio[0], Pio[1], Pio[2], Pio[3]};
+    int it;
+    for (it = 1; it <= n_iter; ++it) {
+        bool ok = c2p_moderate(P[0]) && c2p_moderate(P[1]) && c2p_moderate(P[2]) && c2p_moderate(P[3]);
+        const double gam = d64::root(sq(P[2]) + sq(P[3]) + 1.0);
+        const double w = g * P[1] + P[0];
+        const d64::Div ig = d64::divisor(gam);
+        double f[4], J[16], o[4];
+        f[0] = gam * P[0] - U[0];
+        f[1] = (g - 1.0) * P[1] - sq(gam) * w - U[1];
+        f[2] = P[2] * gam * w - U[2];
+        f[3] = P[3] * gam * w - U[3];
+        J[0] = gam;
+        J[4] = 0.0;
+        J[8] = d64::quot_s(P[0] * P[2], ig);
+        J[12] = d64::quot_s(P[0] * P[3], ig);
+        J[1] = -sq(gam);
+        J[5] = (g - 1.0) - sq(gam) * g;
+        J[9] = -2.0 * P[2] * w;
+        J[13] = -2.0 * P[3] * w;
+        J[2] = gam * P[2];
+        J[6] = gam * P[2] * g;
+        J[10] = d64::quot((2.0 * sq(P[2]) + sq(P[3]) + 1.0), ig) * w;
+        J[14] = d64::quot_s(P[2] * P[3], ig) * w;
+        J[3] = gam * P[3];
+        J[7] = gam * P[3] * g;
+        J[11] = J[14];
+        J[15] = d64::quot((2.0 * sq(P[3]) + sq(P[2]) + 1.0), ig) * w;
+        if (!lu_pivot4_fast(J, f, o, &ok)) return ok ? -1 : C2P_DECLINED;
+        const double s = sq(o[0]) + sq(o[1]) + sq(o[2]) + sq(o[3]);
+        const double norm = d64::is_zero(s) ? s : d64::root(s);
+        if (!(ok && d64::zero_or_in<-900, 900>(s))) return C2P_DECLINED;
+        if (norm < tol) break;
+        P[0] = P[0] - o[0];
+        P[1] = P[1] - o[1];
+        P[2] = P[2] - o[2];
+        P[3] = P[3] - o[3];
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) Pio[v] = P[v];
+    return it;
+}
+
+// Out of line, with the general form inside: inlined into the stage kernels its
+// registers cost more than the call (4096^2 FP64 stage 6.60 against 4.18 ms).
+static __host__ __device__ VB_NOINLINE int c2p_2d(double g, int n_iter, double tol, const double* U, double* P) {
+    const int r = c2p_2d_fast(g, n_iter, tol, U, P);
+    // declined or singular (P is still the guess): from the guess again
+    return r >= 0 ? r : c2p_2d_general(g, n_iter, tol, U, P);
 }
 
 // LU_dec_5D! / LU_dec_2D!, src/3dim/structs.jl:144-214 (no pivoting)
@@ -213,21 +401,15 @@ VB_HD void prims_from_W(double g, double D, double Qx, double Qy, double Qz, dou
     P[4] = qdiv(gm * Qz, W);
 }
 
-#ifdef __CUDA_ARCH__
-#define VB_NOINLINE __noinline__
-#else
-#define VB_NOINLINE
-#endif
-
 static VB_NOINLINE __host__ __device__ int c2p_3d_tail(double g, int n_iter, double tol, const double* Uc, double* P);
 
 // 3D function_UtoP, src/3dim/structs.jl:258-620: 1DW Newton -> Noble 2D
 // Newton with line search -> 5x5 primitive Newton -> bisection. Returns the
 // stage that converged (1..4) or -1 (cell set to NaN, as the reference does).
-// The 1DW stage, which converges for almost every cell, is inline; the rest
-// of the cascade (c2p_3d_tail) is an out-of-line call so that its registers
-// do not count against the stencil kernels.
-VB_HD int c2p_3d(double g, int n_iter, double tol, const double* Uc, double* P) {
+// The rest of the cascade (c2p_3d_tail) is an out-of-line call so that its
+// registers do not count against the stencil kernels.
+static __host__ __device__ VB_NOINLINE int c2p_3d_general(double g, int n_iter, double tol, const double* Uc,
+                                                          double* P) {
     const double D = Uc[0], Q_t = Uc[1], Q_x = Uc[2], Q_y = Uc[3], Q_z = Uc[4];
     double S2, W, v2;
     {
@@ -265,6 +447,78 @@ VB_HD int c2p_3d(double g, int n_iter, double tol, const double* Uc, double* P) 
         }
     }
     return c2p_3d_tail(g, n_iter, tol, Uc, P);
+}
+
+// The 1DW stage, which converges for almost every cell, on the branch-free
+// divide and square root; inline.
+VB_HD int c2p_3d_fast(double g, int n_iter, double tol, const double* Uc, double* P) {
+    const double D = Uc[0], Q_t = Uc[1], Q_x = Uc[2], Q_y = Uc[3], Q_z = Uc[4];
+    const double S2 = Q_x * Q_x + Q_y * Q_y + Q_z * Q_z;
+    if (!(d64::zero_or_in<-550, 200>(S2) && d64::pos_in<-100, 100>(D) && c2p_moderate(Q_x) && c2p_moderate(Q_y) &&
+          c2p_moderate(Q_z) && c2p_moderate(P[2]) && c2p_moderate(P[3]) && c2p_moderate(P[4])))
+        return C2P_DECLINED;
+    const double gm = d64::root(sq(P[2]) + sq(P[3]) + sq(P[4]) + 1.0);
+    const double w_small = P[0] + g * P[1];
+    double W = w_small * sq(gm);
+    const double W_max = 1e30;
+    const double W_min = (d64::is_zero(S2) ? S2 : d64::root(S2)) * (1.0 + 1e-15);
+    const double k = d64::quot(g - 1.0, d64::divisor(g));
+    if (!d64::pos_in<-100, 100>(W)) return C2P_DECLINED;
+    double v2 = d64::quot(S2, d64::divisor(sq(W)));
+    for (int guard = 0; guard < 400 && v2 >= 1.0 && W < W_max; ++guard) {
+        W *= 10.0;
+        v2 = d64::quot(S2, d64::divisor(sq(W)));
+    }
+    for (int it = 0; it < n_iter; ++it) {
+        if (W < W_min) W = W_min;
+        if (!d64::pos_in<-100, 100>(W)) return C2P_DECLINED;
+        v2 = d64::quot(S2, d64::divisor(sq(W)));
+        if (v2 < 0.0)
+            v2 = 0.0;
+        else if (v2 > 1.0 - 1e-15)
+            v2 = 1.0 - 1e-15;
+        const double s = d64::root(1.0 - v2);
+        const double bf = Q_t + W - k * (W * (1.0 - v2) - D * s);
+        const double W3 = W * W * W;
+        const double bj = 1.0 - k * (1.0 - v2) -
+                          k * (W * d64::quot(2.0 * S2, d64::divisor(W3)) - D * d64::quot(S2, d64::divisor(W3 * s)));
+        double dW = d64::quot_s(bf, d64::divisor(bj));
+        if (!(d64::abs_in<-300, 300>(bj) && d64::zero_or_in<-600, 300>(bf))) return C2P_DECLINED;
+        const double Wp = W - dW;
+        if (Wp < W_min)
+            W = 0.5 * (W + W_min);
+        else
+            W = Wp;
+        if (dW < 0) dW = -dW;
+        if (sq(dW) < sq(tol)) {
+            // prims_from_W
+            if (!d64::pos_in<-100, 100>(W)) return C2P_DECLINED;
+            const d64::Div iW = d64::divisor(W);
+            const double a = 1.0 - d64::quot(S2, d64::divisor(sq(W)));
+            if (!d64::pos_in<-60, 1>(a)) return C2P_DECLINED;
+            double lor = d64::quot(1.0, d64::divisor(d64::root(a)));
+            lor = jmin(lor, 50.0);
+            const double Dg = d64::quot(D, d64::divisor(lor));
+            P[0] = jmax(1e-8, Dg);
+            P[1] = jmax(1e-8, d64::quot_s(d64::quot(W, d64::divisor(sq(lor))) - Dg, d64::divisor(g)));
+            P[2] = d64::quot_s(lor * Q_x, iW);
+            P[3] = d64::quot_s(lor * Q_y, iW);
+            P[4] = d64::quot_s(lor * Q_z, iW);
+            return 1;
+        }
+    }
+    return c2p_3d_tail(g, n_iter, tol, Uc, P);
+}
+
+VB_HD int c2p_3d(double g, int n_iter, double tol, const double* Uc, double* P) {
+    const int r = c2p_3d_fast(g, n_iter, tol, Uc, P);
+    if (r != C2P_DECLINED) return r;
+    const double u[5] = {Uc[0], Uc[1], Uc[2], Uc[3], Uc[4]};
+    double p[5] = {P[0], P[1], P[2], P[3], P[4]};
+    const int rg = c2p_3d_general(g, n_iter, tol, u, p);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) P[v] = p[v];
+    return rg;
 }
 
 // Stages 2-4 of the 3D cascade (src/3dim/structs.jl:345-619), entered when

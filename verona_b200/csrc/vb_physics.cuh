@@ -11,6 +11,7 @@
 // ppm32, wenoz32: the same schemes with sign-bit tests, shared differences
 // and approximate reciprocals).
 #pragma once
+#include "vb_fp64.cuh"
 #include "vb_ns.h"
 #include <cuda_runtime.h>
 #include <math.h>
@@ -18,6 +19,11 @@
 #include <string.h>
 
 #define VB_HD __host__ __device__ __forceinline__
+#ifdef __CUDA_ARCH__
+#define VB_NOINLINE __noinline__
+#else
+#define VB_NOINLINE
+#endif
 
 namespace VB_NS {
 
@@ -27,13 +33,23 @@ enum { RS_HLL = 0, RS_HLLC = 1 };
 template <typename T> VB_HD T sq(T x) { return x * x; }
 
 // Base.max / Base.min for IEEE floats: NaN-propagating, +0 > -0.
+// FP64: the upper word of the difference tells a finite one (two finite
+// operands) and its sign, so the NaN tests stay off the FP64 pipe.
 template <typename T> VB_HD T jmax(T x, T y) {
     T d = x - y;
+    if constexpr (sizeof(T) == 8) {
+        const uint32_t h = d64::hi(d);
+        if ((h & 0x7fffffffu) < 0x7ff00000u) return (int32_t)h < 0 ? y : x;
+    }
     if (isnan(x) || isnan(y)) return d;
     return signbit(d) ? y : x;
 }
 template <typename T> VB_HD T jmin(T x, T y) {
     T d = x - y;
+    if constexpr (sizeof(T) == 8) {
+        const uint32_t h = d64::hi(d);
+        if ((h & 0x7fffffffu) < 0x7ff00000u) return (int32_t)h < 0 ? x : y;
+    }
     if (isnan(x) || isnan(y)) return d;
     return signbit(d) ? x : y;
 }
@@ -368,6 +384,151 @@ VB_HD void recon(T q_im2, T q_im1, T q_i, T q_ip1, T q_ip2, T& qr, T& ql) {
         wenoz(q_im2, q_im1, q_i, q_ip1, q_ip2, qr, ql);
 }
 
+// ---- FP64 reconstructions on the branch-free divide (vb_fp64.cuh) -------------
+// The same expressions as wenoz and ppm. They return false where an operand
+// leaves the range in which that divide rounds as the IEEE one; the caller then
+// takes the general form.
+// A product with a power of two is exact, so fma(2, x, y) is the rounded 2 x + y
+// of the expression; 5 x, 7 x and 11 x round by themselves and stay products.
+VB_HD bool wenoz_fast(double q_im2, double q_im1, double q_i, double q_ip1, double q_ip2, double& qr_i,
+                      double& ql_ip1) {
+    const double c1 = 13.0 / 12.0;
+    const double t3 = 3.0 * q_i;
+    const double b1 = fma(0.25, sq(fma(-4.0, q_im1, q_im2 + t3)), c1 * sq(fma(-2.0, q_im1, q_im2 + q_i)));
+    const double b2 = fma(0.25, sq(q_im1 - q_ip1), c1 * sq(fma(-2.0, q_i, q_im1 + q_ip1)));
+    const double b3 = fma(0.25, sq(fma(-4.0, q_ip1, q_ip2 + t3)), c1 * sq(fma(-2.0, q_ip1, q_ip2 + q_i)));
+    const double eps = WenoEps<double>::eps();
+    const double tau5 = fabs(b1 - b3);
+    // Divisors b_k + eps in [2^-140, 2^300] where every b_k < 2^300. A tau5
+    // below 2^-900 may give an inexact ratio, but one below 2^-760, whose square
+    // adds nothing to 1 either way.
+    const double i1 = d64::quot(tau5, d64::divisor(b1 + eps));
+    const double i2 = d64::quot(tau5, d64::divisor(b2 + eps));
+    const double i3 = d64::quot(tau5, d64::divisor(b3 + eps));
+    const double s1 = 1.0 + sq(i1), s2 = 1.0 + sq(i2), s3 = 1.0 + sq(i3);
+    const double m11 = 11.0 * q_i, m5 = 5.0 * q_i;
+    double f1 = fma(2.0, q_im2, -(7.0 * q_im1)) + m11;
+    double f2 = fma(2.0, q_ip1, m5 - q_im1);
+    double f3 = fma(2.0, q_i, 5.0 * q_ip1) - q_ip2;
+    double a1 = 0.1 * s1, a3 = 0.3 * s3;
+    const double a2 = 0.6 * s2;
+    const double nl = f1 * a1 + f2 * a2 + f3 * a3;
+    ql_ip1 = d64::quot_s(nl, d64::divisor(6.0 * (a1 + a2 + a3)));  // divisor in [6, 2^890]
+    f1 = fma(2.0, q_ip2, -(7.0 * q_ip1)) + m11;
+    f2 = fma(2.0, q_im1, m5 - q_ip1);
+    f3 = fma(2.0, q_i, 5.0 * q_im1) - q_im2;
+    a1 = 0.1 * s3;
+    a3 = 0.3 * s1;
+    const double nr = f1 * a1 + f2 * a2 + f3 * a3;
+    qr_i = d64::quot_s(nr, d64::divisor(6.0 * (a1 + a2 + a3)));
+    const uint32_t h1 = d64::hi(b1), h2 = d64::hi(b2), h3 = d64::hi(b3);
+    const uint32_t h12 = h1 > h2 ? h1 : h2, hb = h12 > h3 ? h12 : h3;  // b_k >= 0, or NaN: above every bound
+    // a quotient of at least 2^-800 has a dividend above 2^-800
+    return hb < d64::hi_pow2(300) && (d64::abs_in<-800, 900>(ql_ip1) || d64::is_zero(nl)) &&
+           (d64::abs_in<-800, 900>(qr_i) || d64::is_zero(nr));
+}
+
+// every value zero or in [2^-800, 2^800], so differences are zero or above 2^-860
+VB_HD bool ppm_fast(double q_im2, double q_im1, double q_i, double q_ip1, double q_ip2, double& qr_out,
+                    double& ql_out) {
+    const double C2 = 1.25;
+    double qa = q_i - q_im1;
+    double qb = q_ip1 - q_i;
+    const double dd_im1 = 0.5 * qa + 0.5 * (q_im1 - q_im2);
+    const double dd = 0.5 * qb + 0.5 * qa;
+    const double dd_ip1 = 0.5 * (q_ip2 - q_ip1) + 0.5 * qb;
+    double dph = 0.5 * (q_im1 + q_i) + d64::sixth(dd_im1 - dd);
+    double dph_ip1 = 0.5 * (q_i + q_ip1) + d64::sixth(dd - dd_ip1);
+    const double d2qc_im1 = q_im2 + q_i - 2.0 * q_im1;
+    const double d2qc = q_im1 + q_ip1 - 2.0 * q_i;
+    const double d2qc_ip1 = q_i + q_ip2 - 2.0 * q_ip1;
+
+    double qa_tmp = dph - q_im1;
+    double qb_tmp = q_i - dph;
+    qa = 3.0 * (q_im1 + q_i - 2.0 * dph);
+    double sa = jsign(qa);
+    const double s_m = jsign(d2qc_im1), s_c = jsign(d2qc), s_p = jsign(d2qc_ip1);
+    const double m_m = C2 * fabs(d2qc_im1), m_c = C2 * fabs(d2qc), m_p = C2 * fabs(d2qc_ip1);
+    double qd = sa == s_m && sa == s_c ? sa * jmin(m_m, jmin(m_c, fabs(qa))) : 0.0;
+    const double dph_tmp = 0.5 * (q_im1 + q_i) - d64::sixth(qd);
+    if (qa_tmp * qb_tmp < 0.0) dph = dph_tmp;
+
+    qa_tmp = dph_ip1 - q_i;
+    qb_tmp = q_ip1 - dph_ip1;
+    qa = 3.0 * (q_i + q_ip1 - 2.0 * dph_ip1);
+    sa = jsign(qa);
+    qd = sa == s_c && sa == s_p ? sa * jmin(m_c, jmin(m_p, fabs(qa))) : 0.0;
+    const double dphip1_tmp = 0.5 * (q_i + q_ip1) - d64::sixth(qd);
+    if (qa_tmp * qb_tmp < 0.0) dph_ip1 = dphip1_tmp;
+
+    const double d2qf = 6.0 * (dph + dph_ip1 - 2.0 * q_i);
+    double qr_i = dph, ql_ip1 = dph_ip1;
+    const double dqf_minus = q_i - qr_i, dqf_plus = ql_ip1 - q_i;
+    qa_tmp = dqf_minus * dqf_plus;
+    qb_tmp = (q_ip1 - q_i) * (q_i - q_im1);
+    const double s_f = jsign(d2qf);
+    const double qe = s_m == s_c && s_m == s_p && s_m == s_f
+                          ? s_f * jmin(jmin(m_m, m_c), jmin(m_p, fabs(d2qf)))
+                          : 0.0;
+    qa = jmax(fabs(q_im1), fabs(q_im2));
+    qb = jmax(jmax(fabs(q_i), fabs(q_ip1)), fabs(q_ip2));
+    const bool big = fabs(d2qf) > 1.0e-12 * jmax(qa, qb);
+    const double ratio = d64::quot_s(qe, d64::divisor(d2qf));
+    const double rho = big ? ratio : 0.0;
+    const double tmp_m = q_i - rho * dqf_minus, tmp_p = q_i + rho * dqf_plus;
+    const double tmp2_m = q_i - 2.0 * dqf_plus, tmp2_p = q_i + 2.0 * dqf_minus;
+    if (qa_tmp <= 0.0 || qb_tmp <= 0.0) {
+        if (rho <= 1.0 - 1.0e-12) {
+            qr_i = tmp_m;
+            ql_ip1 = tmp_p;
+        }
+    } else {
+        if (fabs(dqf_minus) >= 2.0 * fabs(dqf_plus)) qr_i = tmp2_m;
+        if (fabs(dqf_plus) >= 2.0 * fabs(dqf_minus)) ql_ip1 = tmp2_p;
+    }
+    qr_out = qr_i;
+    ql_out = ql_ip1;
+    return d64::zero_or_in<-800, 800>(q_im2) && d64::zero_or_in<-800, 800>(q_im1) && d64::zero_or_in<-800, 800>(q_i) &&
+           d64::zero_or_in<-800, 800>(q_ip1) && d64::zero_or_in<-800, 800>(q_ip2);
+}
+
+// the general forms, out of line: reached where wenoz_fast / ppm_fast decline
+template <int REC>
+static __host__ __device__ VB_NOINLINE void recon_general(const double* q, double* out) {
+    recon<REC>(q[0], q[1], q[2], q[3], q[4], out[0], out[1]);
+}
+
+// Reconstruction of N variables of one cell: get(v, o) is variable v of the cell
+// at offset o in [-2, 2] along the axis. FP64: all N through the branch-free
+// forms, whose arithmetic overlaps, then one branch for a variable that needs
+// the general form.
+template <int REC, int N, typename T, typename Get> VB_HD void recon_n(Get get, T* qr, T* ql) {
+    if constexpr (sizeof(T) == 8 && REC != REC_MINMOD) {
+        bool ok = true;
+#pragma unroll
+        for (int v = 0; v < N; ++v) {
+            if constexpr (REC == REC_PPM)
+                ok &= ppm_fast(get(v, -2), get(v, -1), get(v, 0), get(v, 1), get(v, 2), qr[v], ql[v]);
+            else
+                ok &= wenoz_fast(get(v, -2), get(v, -1), get(v, 0), get(v, 1), get(v, 2), qr[v], ql[v]);
+        }
+        if (!ok) {
+#pragma unroll
+            for (int v = 0; v < N; ++v) {
+                const double q[5] = {get(v, -2), get(v, -1), get(v, 0), get(v, 1), get(v, 2)};
+                double o[2];
+                recon_general<REC>(q, o);
+                qr[v] = o[0];
+                ql[v] = o[1];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int v = 0; v < N; ++v)
+            recon<REC>(get(v, -2), get(v, -1), get(v, 0), get(v, 1), get(v, 2), qr[v], ql[v]);
+    }
+}
+
 // a[i] for a runtime axis i < N, as an unrolled select: the arrays of a face
 // state stay in registers, and no access depends on a runtime index (a
 // runtime-indexed local array read back a stale element in one kernel).
@@ -552,12 +713,169 @@ VB_HD void hllc_flux(int d, T g, const T* PL, const T* PR, T* Fo) {
     }
 }
 
+// ---- FP64 face fluxes on the branch-free divide and square root ---------------
+// The same expressions as FaceState, hll_flux and hllc_flux. States with rho, u
+// in [2^-100, 2^100] and velocity components that are zero or in [2^-300, 2^100]
+// keep every divisor, root argument and dividend inside the range of
+// vb_fp64.cuh, except divisors formed by a difference, which are tested where
+// they arise; false is returned for any other state.
+template <int DIM> VB_HD bool face_in_range(const double* P) {
+    bool ok = d64::pos_in<-100, 100>(P[0]) && d64::pos_in<-100, 100>(P[1]);
+#pragma unroll
+    for (int m = 0; m < DIM; ++m) ok = ok && d64::zero_or_in<-300, 100>(P[2 + m]);
+    return ok;
+}
+template <int DIM> struct FaceFast {
+    static constexpr int NV = 2 + DIM;
+    double U[NV], F[NV];
+    double vn, p, lp, lm;
+    VB_HD bool make(int d, double g, const double* P) {
+        double s = sq(P[2]);
+        if (DIM > 1) s = s + sq(P[3]);
+        if (DIM > 2) s = s + sq(P[4]);
+        const double gam = d64::root(s + 1.0);
+        const double w = g * P[1] + P[0];
+        const double un = pick<DIM>(P + 2, d);
+        U[0] = gam * P[0];
+        U[1] = (g - 1.0) * P[1] - sq(gam) * w;
+        F[0] = P[0] * un;
+        F[1] = -w * un * gam;
+#pragma unroll
+        for (int m = 0; m < DIM; ++m) {
+            U[2 + m] = P[2 + m] * gam * w;
+            if (m == d)
+                F[2 + m] = sq(un) * w + (g - 1.0) * P[1];
+            else
+                F[2 + m] = P[2 + m] * un * w;
+        }
+        vn = d64::quot_s(un, d64::divisor(gam));
+        p = (g - 1.0) * P[1];
+        const double C = d64::root(d64::quot((g * (g - 1.0) * P[1]), d64::divisor(P[0] + g * P[1])));
+        const double c1 = 1.0 - sq(C);
+        const double sig = d64::quot(sq(C), d64::divisor(sq(gam) * c1));
+        const double r2 = sig * (1.0 - sq(vn) + sig);
+        const double r = d64::root(r2);
+        const d64::Div is = d64::divisor(1.0 + sig);
+        lp = d64::quot_s(vn + r, is);
+        lm = d64::quot_s(vn - r, is);
+        return d64::pos_in<-60, 60>(c1) && d64::pos_in<-900, 900>(r2);
+    }
+};
+template <int DIM> VB_HD bool hll_fast(int d, double g, const double* PL, const double* PR, double* Fo) {
+    constexpr int NV = 2 + DIM;
+    FaceFast<DIM> R, L;
+    bool ok = face_in_range<DIM>(PL) && face_in_range<DIM>(PR);
+    ok &= R.make(d, g, PR);
+    ok &= L.make(d, g, PL);
+    const double Cmax = jmax(L.lp, R.lp);
+    const double Cmin = -jmin(L.lm, R.lm);
+    const double sum = Cmax + Cmin;
+    const d64::Div is = d64::divisor(sum);
+    const bool use_R = Cmax < 0.0, use_L = !use_R && Cmin < 0.0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const double h = d64::quot_s(R.F[v] * Cmin + L.F[v] * Cmax - Cmax * Cmin * (R.U[v] - L.U[v]), is);
+        Fo[v] = use_R ? R.F[v] : (use_L ? L.F[v] : h);
+    }
+    return ok && (use_R || use_L || d64::pos_in<-300, 300>(sum));
+}
+template <int DIM> VB_HD bool hllc_fast(int d, double g, const double* PL, const double* PR, double* Fo) {
+    constexpr int NV = 2 + DIM;
+    FaceFast<DIM> R, L;
+    bool ok = face_in_range<DIM>(PL) && face_in_range<DIM>(PR);
+    ok &= R.make(d, g, PR);
+    ok &= L.make(d, g, PL);
+    const double Cmax = jmax(L.lp, R.lp);
+    const double Cmin = -jmin(L.lm, R.lm);
+    const double sum = Cmax + Cmin;  // = lR - lL
+    const d64::Div is = d64::divisor(sum);
+    double Fh[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+        Fh[v] = d64::quot_s(R.F[v] * Cmin + L.F[v] * Cmax - Cmax * Cmin * (R.U[v] - L.U[v]), is);
+    const double lL = -Cmin, lR = Cmax;
+    const double idl = d64::quot(1.0, is);
+    const double E_L = -L.U[1], E_R = -R.U[1];
+    const double m_L = pick<DIM>(L.U + 2, d), m_R = pick<DIM>(R.U + 2, d);
+    const double FE_L = -L.F[1], FE_R = -R.F[1];
+    const double Fm_L = pick<DIM>(L.F + 2, d), Fm_R = pick<DIM>(R.F + 2, d);
+    const double E_h = (lR * E_R - lL * E_L - (FE_R - FE_L)) * idl;
+    const double m_h = (lR * m_R - lL * m_L - (Fm_R - Fm_L)) * idl;
+    const double FE_h = (lR * FE_L - lL * FE_R + lR * lL * (E_R - E_L)) * idl;
+    const double Fm_h = (lR * Fm_L - lL * Fm_R + lR * lL * (m_R - m_L)) * idl;
+    const double b = E_h + Fm_h;
+    double disc = b * b - 4.0 * FE_h * m_h;
+    if (disc < 0.0) disc = 0.0;
+    const double rd = d64::root(disc);
+    const double den = b + (d64::is_zero(disc) ? disc : rd);
+    const double ls = d64::quot_s(2.0 * m_h, d64::divisor(den));
+    const double ps = Fm_h - FE_h * ls;
+    const bool left = ls >= 0.0;
+    double U[NV], F[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        U[v] = left ? L.U[v] : R.U[v];
+        F[v] = left ? L.F[v] : R.F[v];
+    }
+    const double lK = left ? lL : lR;
+    const double vn = left ? L.vn : R.vn;
+    const double p = left ? L.p : R.p;
+    const double E = -U[1];
+    const double lks = lK - ls;
+    const d64::Div ik = d64::divisor(lks);
+    const double fac = d64::quot_s(lK - vn, ik);
+    double Us[NV];
+    Us[0] = U[0] * fac;
+#pragma unroll
+    for (int m = 0; m < DIM; ++m)
+        Us[2 + m] = m == d ? d64::quot_s(U[2 + m] * (lK - vn) + ps - p, ik) : U[2 + m] * fac;
+    const double Es = d64::quot_s(E * (lK - vn) + ps * ls - p * vn, ik);
+    Us[1] = -Es;
+    const bool use_R = Cmax < 0.0;
+    const bool use_L = !use_R && Cmin < 0.0;
+    const bool use_hll = !use_R && !use_L && (!(ps > 0.0) || !(ls >= lL && ls <= lR));
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const double fs = F[v] + lK * (Us[v] - U[v]);
+        Fo[v] = use_R ? R.F[v] : (use_L ? L.F[v] : (use_hll ? Fh[v] : fs));
+    }
+    // a supersonic face takes one side's flux whatever the star state is
+    return ok && (use_R || use_L ||
+                  (d64::pos_in<-300, 300>(sum) && d64::abs_in<-300, 300>(den) && d64::abs_in<-300, 300>(lks) &&
+                   d64::zero_or_in<-900, 900>(disc)));
+}
+
 template <int DIM, int RS, typename T>
-VB_HD void face_flux(int d, T g, const T* PL, const T* PR, T* Fo) {
+VB_HD void face_flux_ieee(int d, T g, const T* PL, const T* PR, T* Fo) {
     if (RS == RS_HLLC)
         hllc_flux<DIM>(d, g, PL, PR, Fo);
     else
         hll_flux<DIM>(d, g, PL, PR, Fo);
+}
+template <int DIM, int RS>
+static __host__ __device__ VB_NOINLINE void face_flux_general(int d, double g, const double* PL, const double* PR,
+                                                              double* Fo) {
+    face_flux_ieee<DIM, RS>(d, g, PL, PR, Fo);
+}
+template <int DIM, int RS, typename T>
+VB_HD void face_flux(int d, T g, const T* PL, const T* PR, T* Fo) {
+    if constexpr (sizeof(T) == 8) {
+        const bool ok = RS == RS_HLLC ? hllc_fast<DIM>(d, g, PL, PR, Fo) : hll_fast<DIM>(d, g, PL, PR, Fo);
+        if (!ok) {
+            // copies: the out-of-line call takes addresses, the fast path's states stay in registers
+            double l[2 + DIM], r[2 + DIM], f[2 + DIM];
+#pragma unroll
+            for (int v = 0; v < 2 + DIM; ++v) {
+                l[v] = PL[v];
+                r[v] = PR[v];
+            }
+            face_flux_general<DIM, RS>(d, g, l, r, f);
+#pragma unroll
+            for (int v = 0; v < 2 + DIM; ++v) Fo[v] = f[v];
+        }
+    } else {
+        face_flux_ieee<DIM, RS>(d, g, PL, PR, Fo);
+    }
 }
 
 // Largest |lambda| over the axes of one cell-centred state (CFL signal speed;

@@ -93,7 +93,9 @@ static __device__ __noinline__ int solve_cell_learned(const StageParams& p, cons
 // from a supplied guess with the bracketed fallback.
 // MODE: 0 reads p.c2p_mode at run time; 1 (reference) and 2 (W Newton) fix
 // it at compile time, so a kernel of one mode carries no code of the other.
-template <int DIM, int MODE = 0>
+// CALL: the 1D Newton out of line too (kernels whose W Newton leaves it only the
+// fallback cells, whose registers it would otherwise take).
+template <int DIM, int MODE = 0, bool CALL = false>
 __device__ __forceinline__ int solve_cell(const StageParams& p, const double* U, double* P, long long gidx,
                                           int& fallback, int* fp64 = nullptr) {
     fallback = 0;
@@ -140,7 +142,10 @@ __device__ __forceinline__ int solve_cell(const StageParams& p, const double* U,
         auto ref_try = [&](int& r) -> bool {
 #pragma unroll
             for (int v = 0; v < 2 + DIM; ++v) P[v] = Pin[v];
-            r = DIM == 1 ? c2p_1d(p.gamma, p.n_iter, p.tol, U, P) : c2p_2d(p.gamma, p.n_iter, p.tol, U, P);
+            if constexpr (DIM == 1)
+                r = CALL ? c2p_1d_call(p.gamma, p.n_iter, p.tol, U, P) : c2p_1d(p.gamma, p.n_iter, p.tol, U, P);
+            else
+                r = c2p_2d(p.gamma, p.n_iter, p.tol, U, P);
             bool finite = true;
 #pragma unroll
             for (int v = 0; v < 2 + DIM; ++v) finite = finite && isfinite(P[v]);
@@ -319,7 +324,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs
         auto recon_var = [&](int v, int base, int fR, int fL, bool wR, bool wL) {
             const R* q = sP + v * EXT + base;
             R qr, ql;
-            recon<REC>(q[-2 * sd], q[-sd], q[0], q[sd], q[2 * sd], qr, ql);
+            recon_n<REC, 1, R>([&](int, int o) { return q[o * sd]; }, &qr, &ql);
             if (v < 2) {
                 qr = jmax(fl, qr);
                 ql = jmax(fl, ql);
@@ -331,8 +336,18 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs
             int base, fR, fL;
             bool wR, wL;
             if (!cell_at(e % TX, (e / TX) % TY, e / (TX * TY), base, fR, fL, wR, wL)) continue;
+            R qr[NV], ql[NV];
+            const R* q = sP + base;
+            recon_n<REC, NV, R>([&](int v, int o) { return q[v * EXT + o * sd]; }, qr, ql);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) recon_var(v, base, fR, fL, wR, wL);
+            for (int v = 0; v < NV; ++v) {
+                if (v < 2) {
+                    qr[v] = jmax(fl, qr[v]);
+                    ql[v] = jmax(fl, ql[v]);
+                }
+                if (wR) sR[v * NF + fR] = qr[v];
+                if (wL) sL[v * NF + fL] = ql[v];
+            }
         }
         {
             // halo layers c_d = -1 and c_d = T_d: (cell, variable) items, variable-major
@@ -405,7 +420,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs
         }
         if (p.skip_c2p) continue;  // con2prim runs in a separate kernel
         int fb;
-        int r = solve_cell<DIM>(p, U, P, gidx, fb);
+        int r = solve_cell<DIM, 0, CG && sizeof(R) == 4>(p, U, P, gidx, fb);
         n_fail += (r < 0);
         n_fb += fb;
         n_it += (r < 0 ? -r : r);

@@ -70,10 +70,20 @@ template <> struct DivAcc<float> {
 
 template <int REC, typename R>
 __device__ __forceinline__ void recon_floored(const R* q, int s, R fl, int v, R& qr, R& ql) {
-    recon<REC>(q[-2 * s], q[-s], q[0], q[s], q[2 * s], qr, ql);
+    recon_n<REC, 1, R>([&](int, int o) { return q[o * s]; }, &qr, &ql);
     if (v < 2) {  // face floor of rho and u (src/3dim/algos.jl:112-115)
         qr = jmax(fl, qr);
         ql = jmax(fl, ql);
+    }
+}
+// every variable of one cell; the variables' planes are `pln` apart
+template <int REC, typename R>
+__device__ __forceinline__ void recon_cell_floored(const R* q, int s, int pln, R fl, R* qr, R* ql) {
+    recon_n<REC, 5, R>([&](int v, int o) { return q[v * pln + o * s]; }, qr, ql);
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        qr[v] = jmax(fl, qr[v]);
+        ql[v] = jmax(fl, ql[v]);
     }
 }
 
@@ -115,14 +125,11 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
         for (int v = 0; v < NV; ++v) zslot(z, v) = b.Pin[v * vs + col + sz * z];
     };
     auto zrecon = [&](int zc, R* qr, R* ql) {  // reconstruct cell zc along z, floored
+        recon_n<REC, NV, R>([&](int v, int o) { return zslot(zc + o, v); }, qr, ql);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            recon<REC>(zslot(zc - 2, v), zslot(zc - 1, v), zslot(zc, v), zslot(zc + 1, v), zslot(zc + 2, v), qr[v],
-                       ql[v]);
-            if (v < 2) {
-                qr[v] = jmax(fl, qr[v]);
-                ql[v] = jmax(fl, ql[v]);
-            }
+        for (int v = 0; v < 2; ++v) {
+            qr[v] = jmax(fl, qr[v]);
+            ql[v] = jmax(fl, ql[v]);
         }
     };
     R qlz[NV];  // left state of face k+1/2 (ql of cell k)
@@ -169,14 +176,10 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
         // x: reconstruct own cell; halo cells -1 and TX of each row
         R qrx[NV];
         {
-            const R* q = sPl + (ty + 3) * EX + tx + 3;
+            R ql[NV];
+            recon_cell_floored<REC>(sPl + (ty + 3) * EX + tx + 3, 1, PLN, fl, qrx, ql);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                R qr, ql;
-                recon_floored<REC>(q + v * PLN, 1, fl, v, qr, ql);
-                qrx[v] = qr;
-                sQL[v * FN + ty * FXR + tx + 1] = ql;
-            }
+            for (int v = 0; v < NV; ++v) sQL[v * FN + ty * FXR + tx + 1] = ql[v];
         }
         // the x halo as (cell, variable) items, on the last threads (the first
         // ones take the y halo): one variable's reconstruction each instead of
@@ -229,14 +232,10 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_stage_zm(StageParams p, Stage
         // y: reconstruct own cell; halo cells -1 and TY of each column
         R qry[NV];
         {
-            const R* q = sPl + (ty + 3) * EX + tx + 3;
+            R ql[NV];
+            recon_cell_floored<REC>(sPl + (ty + 3) * EX + tx + 3, EX, PLN, fl, qry, ql);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                R qr, ql;
-                recon_floored<REC>(q + v * PLN, EX, fl, v, qr, ql);
-                qry[v] = qr;
-                sQL[v * FN + (ty + 1) * TX + tx] = ql;
-            }
+            for (int v = 0; v < NV; ++v) sQL[v * FN + (ty + 1) * TX + tx] = ql[v];
         }
         __syncthreads();
         {
@@ -382,9 +381,13 @@ inline dim3 z_march_grid(const StageParams& p, int TX, int TY, int ctas_per_sm, 
 
 // Split-mode con2prim: one thread per interior cell, no barriers, no shared
 // memory; reads the stage's U and the guess (the stage's input P, or the
-// per-cell W guesses of p.w_guess), writes the floored P.
+// per-cell W guesses of p.w_guess), writes the floored P. The reference cascade
+// (MODE 1) is bound by its serial Newton and its loads, so it takes 64 registers
+// and 8 x 128 threads per SM: 4.2 M cells, FP32 P, 143 us (floor by its 80 bytes
+// a cell 52 us); 175 us at 128 registers, 210 us with the IEEE divides.
+template <int MODE> struct C2pCfg { static constexpr int NT = MODE == 1 ? 128 : 256, MINB = MODE == 1 ? 8 : 1; };
 template <typename R, int MODE>
-__global__ void __launch_bounds__(256) k_c2p(StageParams p, StageBufs<R> b) {
+__global__ void __launch_bounds__(C2pCfg<MODE>::NT, C2pCfg<MODE>::MINB) k_c2p(StageParams p, StageBufs<R> b) {
     constexpr int NV = 5;
     const int N0 = p.n[0] - 2 * NG, N1 = p.n[1] - 2 * NG, N2 = p.n[2] - 2 * NG;
     const long long tot = (long long)N0 * N1 * N2;  // < 2^32 (launch_c2p)
@@ -436,8 +439,11 @@ __global__ void __launch_bounds__(256) k_c2p(StageParams p, StageBufs<R> b) {
 // The same for a 2D grid (padded extents (Nx + 6, Ny + 6, 1)): one thread per
 // interior cell, the reference's 2D con2prim (solve_cell<2>) from the stage's
 // input P, floors, P out; the statistics as the fused box kernel counts them.
-template <typename R>
-__global__ void __launch_bounds__(256) k_c2p_2d(StageParams p, StageBufs<R> b) {
+// MODE as k_c2p's: 1 the reference, 6 x 128 threads per SM (80 registers): 4096^2
+// FP64 1.56 ms, against 2.43 ms at 149 registers, 1.67 at 8 x 128; 2 the W Newton.
+template <int MODE> struct C2p2dCfg { static constexpr int NT = MODE == 1 ? 128 : 256, MINB = MODE == 1 ? 6 : 1; };
+template <typename R, int MODE>
+__global__ void __launch_bounds__(C2p2dCfg<MODE>::NT, C2p2dCfg<MODE>::MINB) k_c2p_2d(StageParams p, StageBufs<R> b) {
     constexpr int NV = 4;
     const int N0 = p.n[0] - 2 * NG, N1 = p.n[1] - 2 * NG;
     const long long tot = (long long)N0 * N1;  // < 2^32 (launch_c2p)
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(256) k_c2p_2d(StageParams p, StageBufs<R> b) {
         }
         int fb;
         int r;
-        if (p.c2p_mode == C2P_GUESS_W) {
+        if constexpr (MODE == 2) {
             // the previous state's W (VB_GUESS_PREVIOUS_W): the W Newton of the
             // 3D scheme on the state padded to three momenta (u^z = 0), with
             // the precision gate of the FP32-bulk form. It runs only here,
@@ -507,15 +513,18 @@ template <typename R> cudaError_t launch_c2p(const StageParams& p, const StageBu
     if (p.n[2] == 1) {
         const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG);
         if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
-        k_c2p_2d<R><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
+        if (p.c2p_mode == C2P_GUESS_W)
+            k_c2p_2d<R, 2><<<grid_for(cells, C2p2dCfg<2>::NT), C2p2dCfg<2>::NT, 0, s>>>(p, b);
+        else
+            k_c2p_2d<R, 1><<<grid_for(cells, C2p2dCfg<1>::NT), C2p2dCfg<1>::NT, 0, s>>>(p, b);
         return cudaGetLastError();
     }
     const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG) * (p.n[2] - 2 * NG);
     if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
     if (p.c2p_mode == C2P_GUESS_W)
-        k_c2p<R, 2><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
+        k_c2p<R, 2><<<grid_for(cells, C2pCfg<2>::NT), C2pCfg<2>::NT, 0, s>>>(p, b);
     else
-        k_c2p<R, 1><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
+        k_c2p<R, 1><<<grid_for(cells, C2pCfg<1>::NT), C2pCfg<1>::NT, 0, s>>>(p, b);
     return cudaGetLastError();
 }
 
@@ -541,13 +550,7 @@ cudaError_t launch_stage_zm_t(const StageParams& p, const StageBufs<R>& b, cudaS
     kern<<<grid, C::TX * C::TY, smem, s>>>(p, b, lz);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !SPLIT || p.skip_c2p) return e;
-    const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG) * (p.n[2] - 2 * NG);
-    if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
-    if (p.c2p_mode == C2P_GUESS_W)
-        k_c2p<R, 2><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
-    else
-        k_c2p<R, 1><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
-    return cudaGetLastError();
+    return launch_c2p<R>(p, b, s);
 }
 
 template <int REC, int RS, typename R>

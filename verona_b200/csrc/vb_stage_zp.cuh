@@ -904,13 +904,7 @@ cudaError_t launch_stage_zp_g(const StageParams& p, const StageBufs<float>& b, d
     kern<<<grid, C::TX * C::TY, smem, s>>>(p, b, lz, tm);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || TAIL != ZP_U || p.skip_c2p) return e;
-    const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG) * (p.n[2] - 2 * NG);
-    if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
-    if (p.c2p_mode == C2P_GUESS_W)
-        k_c2p<float, 2><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
-    else
-        k_c2p<float, 1><<<grid_for(cells, 256), 256, 0, s>>>(p, b);
-    return cudaGetLastError();
+    return launch_c2p<float>(p, b, s);
 }
 
 template <int REC, int RS, int TAIL, bool TMA>
