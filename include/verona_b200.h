@@ -221,13 +221,15 @@ int vb_reset_counters(vb_handle h, void* stream);
  * the W Newton from it run in one kernel; 0 = a guess kernel writes one W per
  * cell and the con2prim kernel reads it; -1 = library default (1). Both start
  * the Newton from the same FP32-rounded guess.
- * fp32_pairs (precision = VB_PREC_FP32_BULK, 3D, every reconstruction with HLL or HLLC): 1 =
- * the z-pair stencil kernel (two cells per thread on packed FP32 pairs);
- * 0 = one cell per thread; -1 = library default (1). The two agree to FP32
- * rounding, not bitwise.
+ * fp32_pairs (precision = VB_PREC_FP32_BULK, 2D and 3D, every reconstruction with HLL or HLLC):
+ * 1 = the z-pair (3D) or y-marching (2D) stencil kernel, two cells per thread on
+ * packed FP32 pairs (in 2D con2prim then runs in a kernel of its own, whatever
+ * split_con2prim); 0 = one cell per thread; -1 = library default (1). The two
+ * agree to FP32 rounding, not bitwise.
  * tma_tiles: 1 = the stencil kernels stage the state in shared memory as TMA
  * tiles (cp.async.bulk.tensor): in 3D (FP32 bulk, z-pair kernel) every plane
- * with its x/y halo, a ring of 6 planes per CTA; in 2D (both precisions) the
+ * with its x/y halo, a ring of 6 planes per CTA; in 2D FP32 bulk every row of a
+ * warp's strip, a ring of 8 rows; in 2D FP64 (and FP32 with fp32_pairs = 0) the
  * CTA's tile with its halo on both axes; 0 = staged by per-thread loads (3D:
  * the thread's own column, 4-byte asynchronous copies for the halo);
  * -1 = library default (1). Results are identical.

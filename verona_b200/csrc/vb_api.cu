@@ -59,6 +59,8 @@ struct vb_solver {
     // TMA tensor maps of P[0], P[1] (the TMA forms of the stage kernels: 3D FP32, 2D)
     alignas(64) unsigned char tmap[2][128] = {};
     bool tmap_ok[2] = {false, false};
+    alignas(64) unsigned char tmap_row[2][128] = {};  // by rows (2D FP32)
+    bool tmap_row_ok[2] = {false, false};
     // learned con2prim guess
     const void* mlp_blob = nullptr;
     unsigned int* tc_err = nullptr;
@@ -252,9 +254,12 @@ int vb_create(vb_handle* out, int dims, int nx, int ny, int nz, int nghost, cons
         }
     }
     if (nghost != 0 && dims >= 2)
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 2; ++i) {
+            h->tmap_row_ok[i] =
+                dims == 2 && fp32(h) && encode_stage_row_tmap(h->tmap_row[i], (const float*)h->P[i], grid_of(h));
             h->tmap_ok[i] = fp32(h) ? encode_stage_tmap<float>(h->tmap[i], (const float*)h->P[i], grid_of(h))
                                     : encode_stage_tmap<double>(h->tmap[i], (const double*)h->P[i], grid_of(h));
+        }
     h->max_partial = max_speed_blocks(grid_of(h));
     if ((rc = dev_alloc(h, (void**)&h->cnt, sizeof(unsigned long long) * CNT_N)) ||
         (rc = dev_alloc(h, (void**)&h->partial, sizeof(double) * (h->max_partial + 1)))) {
@@ -588,9 +593,12 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
         return fail(h, VB_ERR_STATE, "vb_step: FMA-contracted FP64 unit built from another StageParams");
     auto stage = [&](const R* Pin, R* Pout, const double* Us, double* Uo, double dts, double a, double b) -> int {
         for (int d = 0; d < 3; ++d) p.dtdx[d] = d < h->dims ? dts / h->dx[d] : 0.0;
-        p.tmap_in = nullptr;
-        for (int i = 0; i < 2; ++i)
-            if (tma && h->tmap_ok[i] && (const void*)Pin == h->P[i]) p.tmap_in = h->tmap[i];
+        p.tmap_in = p.tmap_row = nullptr;
+        for (int i = 0; i < 2; ++i) {
+            if (!tma || (const void*)Pin != h->P[i]) continue;
+            if (h->tmap_ok[i]) p.tmap_in = h->tmap[i];
+            if (h->tmap_row_ok[i]) p.tmap_row = h->tmap_row[i];
+        }
         p.rk_a = a;
         p.rk_b = b;
         StageBufs<R> bufs{Pin, Pout, h->U0, Us, Uo};
@@ -819,7 +827,9 @@ int vb_get_tuning(vb_handle h, vb_tuning* t) {
 
 int vb_tma_tiles_active(vb_handle h, int* active) {
     if (!h || !active) return fail(h, VB_ERR_ARG, "vb_tma_tiles_active: null argument");
-    *active = h->tun.tma_tiles != 0 && h->tmap_ok[0] && h->tmap_ok[1] ? 1 : 0;
+    const bool rows = h->dims == 2 && fp32(h) && h->tun.fp32_pairs != 0;  // y-marching kernel
+    const bool* ok = rows ? h->tmap_row_ok : h->tmap_ok;
+    *active = h->tun.tma_tiles != 0 && ok[0] && ok[1] ? 1 : 0;
     return VB_OK;
 }
 

@@ -45,12 +45,14 @@ struct StageParams {
     int force_box;       // 1: use the box-tile kernel even where the z-marching one fits
     int split;           // 1: z-marching stencil kernel writes U only; k_c2p solves con2prim
     int skip_c2p;        // 1: the stencil kernel writes U only and launches no con2prim
-    int pairs;           // 1: FP32-bulk 3D stages use the z-pair kernel where it exists
+    int pairs;           // 1: FP32-bulk 3D / 2D stages use the z-pair / y-marching kernel (two cells per thread)
     int div_in_pout;     // 1: the stencil kernel left the FP32 divergence in Pout; the
                          //    con2prim kernel forms Uo = rk_a U0 + rk_b (Us - div) itself
     int want_div;        // 1: the caller's con2prim kernel (skip_c2p) accepts div_in_pout
     int c2p_rescue;      // 1: 1D / 2D cells whose reference Newton diverges are solved by the
                          //    bracketed W Newton (batched problems); 0: kept and counted as failures
+    const void* tmap_row; // host CUtensorMap of Pin by rows (encode_stage_row_tmap), for the TMA form of
+                          //    the y-marching 2D kernel; nullptr: rows staged by asynchronous copies
     const void* tmap_in; // host CUtensorMap of Pin (encode_stage_tmap) for the TMA forms: the 3D
                          //    z-pair kernel's planes, k_stage's 2D tiles; nullptr: staged by loads
 };
@@ -124,6 +126,10 @@ int max_speed_blocks(const Grid& g);
 // vb_stage_f32.cu): WENOZ reconstruction with HLL or HLLC
 inline bool zp_available(int rec, int rs) { return rec >= 0 && rec <= 2 && (rs == 0 || rs == 1); }
 cudaError_t launch_stage_zp(int rec, int rs, const StageParams& p, const StageBufs<float>& b, cudaStream_t s);
+// the y-marching 2D stage of the FP32-bulk form (vb_stage_yp.cuh, p.pairs): writes U, no con2prim
+cudaError_t launch_stage_yp(int rec, int rs, const StageParams& p, const StageBufs<float>& b, cudaStream_t s);
+// tensor map of one 2D FP32 state array by rows, for its TMA form (p.tmap_row)
+bool encode_stage_row_tmap(void* out, const float* P, const Grid& g);
 // tensor map of one SoA state array for the TMA forms of the stage kernels
 // (3D FP32: the z-pair kernel's plane boxes; 2D: k_stage's tile boxes; out: a
 // 64-byte aligned CUtensorMap); false where no TMA form exists or the layout

@@ -511,8 +511,8 @@ cudaError_t dispatch_stage_dim(int rec, int rs, const StageParams& p, const Stag
 template <typename R>
 cudaError_t dispatch_stage_zm(int rec, int rs, const StageParams& p, const StageBufs<R>& b, cudaStream_t s);
 
-// 3D grids use the z-marching kernels (unless force_box); 1D and 2D the
-// box-tile k_stage.
+// 3D grids use the z-marching kernels (unless force_box) and 2D FP32-bulk grids
+// the y-marching one (unless pairs = 0); 1D and 2D FP64 the box-tile k_stage.
 // *kernels receives the number of kernels launched (2 for a split z-march
 // stage, whose con2prim runs in k_c2p; else 1).
 template <typename R>
@@ -521,6 +521,15 @@ cudaError_t launch_stage(int dims, int rec, int rs, const StageParams& p, const 
     *kernels = 1;
     if (dims == 1) return dispatch_stage_dim<1, R>(rec, rs, p, b, s);
     if (dims == 2) {
+        if constexpr (sizeof(R) == 4) {
+            // the y-marching kernel, which writes U, then k_c2p_2d
+            if (p.pairs) {
+                const cudaError_t e = launch_stage_yp(rec, rs, p, b, s);
+                if (e != cudaSuccess || p.skip_c2p) return e;
+                *kernels = 2;
+                return launch_c2p<R>(p, b, s);
+            }
+        }
         if (!p.split || p.skip_c2p) return dispatch_stage_dim<2, R>(rec, rs, p, b, s);
         // split: the box kernel writes U only, then k_c2p_2d
         StageParams q = p;

@@ -569,7 +569,10 @@ template <typename R> int stage_div_in_pout(int dims, int rec, int rs, const Sta
 // launches result from launch_stage with skip_c2p = 1, want_div = 0 followed
 // by launch_c2p
 template <typename R> int stage_split_c2p(int dims, const StageParams& p) {
-    if (dims == 2) return p.split && !p.skip_c2p ? 1 : 0;
+    if (dims == 2) {
+        const bool yp = std::is_same<R, float>::value && p.pairs;
+        return (p.split || yp) && !p.skip_c2p ? 1 : 0;
+    }
     return dims == 3 && !p.force_box && p.split && !p.skip_c2p ? 1 : 0;
 }
 

@@ -75,6 +75,11 @@ __device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
                  "l"(gsrc)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(sdst)),
+                 "l"(gsrc)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ f2 sel(m2 m, f2 a, f2 b) { return P2(m.x ? a.x : b.x, m.y ? a.y : b.y); }
 
@@ -251,17 +256,22 @@ __device__ __forceinline__ void recon2(f2 qm2, f2 qm1, f2 q0, f2 qp1, f2 qp2, f2
     }
 }
 
-// One face state along axis D (compile time): the primitive state and what
-// the HARM speeds / HLL / HLLC need from it (src/3dim/algos.jl:117-157).
-// Sign convention of the energy slot: E = -U[1] > 0 and FE = -F[1].
-template <int D> struct Side {
-    f2 P[5];
+// One face state of a DIM-dimensional grid along axis D (compile time): the
+// primitive state and what the HARM speeds / HLL / HLLC need from it
+// (src/3dim/algos.jl:117-157). Sign convention of the energy slot: E = -U[1] > 0
+// and FE = -F[1].
+template <int D, int DIM = 3> struct Side {
+    static constexpr int NV = 2 + DIM;
+    f2 P[NV];
     f2 gam, gw, uw, vn, p, np, lp, lm;
     __device__ __forceinline__ void make(f2 g, f2 gm1, const f2* Pin) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) P[v] = Pin[v];
+        for (int v = 0; v < NV; ++v) P[v] = Pin[v];
         const f2 one = S2(1.0f);
-        gam = vsqrt(fma(P[4], P[4], fma(P[3], P[3], fma(P[2], P[2], one))));
+        f2 g2 = fma(P[2], P[2], one);
+#pragma unroll
+        for (int v = 3; v < NV; ++v) g2 = fma(P[v], P[v], g2);
+        gam = vsqrt(g2);
         const f2 w = fma(g, P[1], P[0]);
         const f2 un = P[2 + D];
         gw = mul(gam, w);
@@ -299,9 +309,10 @@ template <int D> struct Side {
 
 // HLL (RS_HLL, src/3dim/algos.jl:149-174) or HLLC (RS_HLLC: Mignone & Bodo
 // 2005 with the HLL fallback for an unphysical star state) flux of two faces.
-template <int D, int RS>
+template <int D, int RS, int DIM = 3>
 __device__ __forceinline__ void face_flux(f2 g, f2 gm1, const f2* PL, const f2* PR, f2* Fo) {
-    Side<D> L, R;
+    constexpr int NV = 2 + DIM;
+    Side<D, DIM> L, R;
     L.make(g, gm1, PL);
     R.make(g, gm1, PR);
     const f2 lR = vmax(L.lp, R.lp);  // Cmax
@@ -313,13 +324,13 @@ __device__ __forceinline__ void face_flux(f2 g, f2 gm1, const f2* PL, const f2* 
     const f2 nlL = mul(S2(-1.0f), lL);
     const f2 cL = mul(lR, idl), cR = mul(nlL, idl), cU = mul(mul(lR, lL), idl);
     auto hll = [&](int v) { return fma(cU, sub(R.U(v), L.U(v)), fma(cL, L.F(v), mul(cR, R.F(v)))); };
-    f2 Fh[5];
+    f2 Fh[NV];
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
+    for (int v = 0; v < NV; ++v)
         if (RS == RS_HLL || v == 1 || v == 2 + D) Fh[v] = hll(v);
     if (RS == RS_HLL) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) {
+        for (int v = 0; v < NV; ++v) {
             f2 o = sel(use_R, R.F(v), sel(use_L, L.F(v), Fh[v]));
             Fo[v] = v == 1 ? mul(S2(-1.0f), o) : o;
         }
@@ -356,7 +367,7 @@ __device__ __forceinline__ void face_flux(f2 g, f2 gm1, const f2* PL, const f2* 
     const f2 lkfS = P2(sup.x ? 0.0f : lkf.x, sup.y ? 0.0f : lkf.y);
     const bool any_hll = use_hll.x || use_hll.y;
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
+    for (int v = 0; v < NV; ++v) {
         f2 o;
         if (v == 1 || v == 2 + D) {
             const f2 UK = sel(left, L.U(v), R.U(v));
@@ -377,7 +388,7 @@ __device__ __forceinline__ void face_flux(f2 g, f2 gm1, const f2* PL, const f2* 
     }
     if (any_hll) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v)
+        for (int v = 0; v < NV; ++v)
             if (v != 1 && v != 2 + D) Fo[v] = sel(use_hll, hll(v), Fo[v]);
     }
 }
