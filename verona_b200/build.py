@@ -1,7 +1,7 @@
 """Build libverona_b200.so in-tree with nvcc for sm_100a.
 
 Translation units and their floating-point contract:
-  vb_stage_f64.cu, vb_ref1d.cu, vb_api.cu  -fmad=false  (FP64 path rounds as
+  vb_stage_f64.cu, vb_ref1d.cu, vb_tube.cu, vb_api.cu  -fmad=false  (FP64 path rounds as
                                             the reference: no FMA contraction)
   vb_stage_f64c.cu                          -fmad=true   (the FP64 stage kernels with FMA
                                             contraction, namespace vb_f64c; tuning
@@ -36,6 +36,7 @@ UNITS = {
     "vb_stage_f64.cu": ["-fmad=false"],
     "vb_stage_f64c.cu": ["-fmad=true"],
     "vb_ref1d.cu": ["-fmad=false"],
+    "vb_tube.cu": ["-fmad=false"],
     "vb_api.cu": ["-fmad=false"],
     "vb_stage_f32.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
     "vb_stage_yp_f32.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],

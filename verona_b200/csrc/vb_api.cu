@@ -11,6 +11,7 @@
 //   stage  FP64 AoS staging buffer for host-pointer loads/stores (lazy)
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -20,6 +21,7 @@
 
 #include "../../include/verona_b200.h"
 #include "vb_internal.h"
+#include "vb_tube.h"
 
 using namespace vb;
 
@@ -680,6 +682,44 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
     return VB_OK;
 }
 
+// launch_tube's steps, at most TUBE_STEPS a launch; VB_ERR_UNSUPPORTED (nothing done) where it is refused
+static int step_tube(vb_handle h, double dt, int nsteps, cudaStream_t s) {
+    constexpr int TUBE_STEPS = 4096;
+    StageParams p{};
+    for (int a = 0; a < 3; ++a) p.n[a] = h->np[a];
+    p.sy = h->sy;
+    p.sz = h->sz;
+    p.vs = h->vs;
+    p.gamma = h->gamma;
+    p.floor_ = h->opt.floor_;
+    p.tol = h->opt.tol;
+    p.n_iter = h->opt.n_iter;
+    p.stats = h->opt.stats;
+    p.c2p_mode = C2P_REFERENCE;
+    p.counters = h->cnt;
+    while (nsteps > 0) {
+        TubeRun r{};
+        for (int i = 0; i < 2; ++i) r.P[i] = (double*)h->P[i];
+        r.U0 = h->U0;
+        r.U1 = h->U1;
+        r.cur = h->cur;
+        r.rk = h->opt.rk;
+        r.nsteps = std::min(nsteps, TUBE_STEPS);
+        r.t0 = h->t;
+        r.dt = dt;
+        r.dtdx = dt / h->dx[0];
+        r.half_dtdx = (dt / 2) / h->dx[0];
+        const cudaError_t e = launch_tube(h->opt.recon, h->opt.riemann, r, h->bc_kind, h->bc_par, p, s);
+        if (e == cudaErrorNotSupported) return VB_ERR_UNSUPPORTED;  // the first launch's answer, if any
+        if (e != cudaSuccess) return fail(h, VB_ERR_CUDA, "launch_tube: %s", cudaGetErrorString(e));
+        h->launches += 1;
+        for (int n = 0; n < r.nsteps; ++n) h->t += dt;
+        if (h->opt.rk == 3 && (r.nsteps & 1)) h->cur = 1 - h->cur;
+        nsteps -= r.nsteps;
+    }
+    return VB_OK;
+}
+
 extern "C" {
 
 int vb_step(vb_handle h, double dt, int nsteps, void* stream) {
@@ -693,6 +733,11 @@ int vb_step(vb_handle h, double dt, int nsteps, void* stream) {
         h->launches += 1;
         for (int n = 0; n < nsteps; ++n) h->t += dt;
         return VB_OK;
+    }
+    // a short 1D FP64 grid: all steps in one launch (not while the stages are timed one by one)
+    if (h->dims == 1 && !fp32(h) && !h->prof && h->tun.fp64_contract != 1 && nsteps > 0 && tube_fits(h->n[0])) {
+        const int rc = step_tube(h, dt, nsteps, s);
+        if (rc != VB_ERR_UNSUPPORTED) return rc;
     }
     for (int n = 0; n < nsteps; ++n) {
         int rc = fp32(h) ? step_nd<float>(h, dt, s) : step_nd<double>(h, dt, s);

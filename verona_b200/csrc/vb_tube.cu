@@ -1,0 +1,130 @@
+// Ghosted 1D grids of up to 2048 cells, FP64: every step of a call in one launch
+// of a thread-block cluster. One CTA per 128-cell tile runs the box tile's stage
+// body (stage_tile, vb_stage.cuh) with its loads past L1, edge tiles fill and
+// floor their ghosts as the batch kernel does (batch_ghosts), and the cluster
+// meets once per stage. The kernels of one stage take about as long to launch as
+// to run at this size: N = 1024, MINMOD + HLLC, RK2, 10 steps 377 us in 60 launches,
+// 158 us in one. Longer grids fill the GPU from separate launches and keep
+// them. Built with -fmad=false: the same arithmetic as those kernels, bit for bit.
+#include <algorithm>
+#include <cstring>
+
+#include "vb_batch.cuh"
+#include "vb_tube.h"
+
+namespace vb {
+
+constexpr int TUBE_TX = 128, TUBE_CLUSTER = 16;
+
+__device__ __forceinline__ void tube_meet() {
+    __threadfence();  // this thread's stores before the other CTAs' loads
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int REC, int RS>
+__global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, BatchProb pr, StageParams q) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double t = r.t0;
+    int c = r.cur;
+    const int stages = r.rk == 3 ? 3 : 2;
+    const bool short_last = pr.ntx > 1 && (pr.n0 - 2 * NG) - (pr.ntx - 1) * TUBE_TX < NG;
+    for (int n = 0; n < r.nsteps; ++n, t += r.dt) {
+        double *Pc = r.P[c], *Pn = r.P[1 - c];
+        for (int st = 0; st < stages; ++st) {
+            StageBufs<double> b;
+            b.Pin = (st & 1) ? Pn : Pc;
+            b.Pout = (st & 1) ? Pc : Pn;
+            b.U0 = r.U0;
+            q.dtdx[0] = r.rk == 2 && st == 0 ? r.half_dtdx : r.dtdx;
+            if (r.rk == 3) {  // SSP-RK3
+                q.rk_a = st == 0 ? 0.0 : (st == 1 ? 0.75 : 1.0 / 3.0);
+                q.rk_b = st == 0 ? 1.0 : (st == 1 ? 0.25 : 2.0 / 3.0);
+                b.Us = st == 0 ? r.U0 : r.U1;
+                b.Uo = st == 2 ? r.U0 : r.U1;
+            } else {  // midpoint RK2
+                q.rk_a = 0.0;
+                q.rk_b = 1.0;
+                b.Us = r.U0;
+                b.Uo = st ? r.U0 : r.U1;
+            }
+            const int tile = (int)blockIdx.x;
+            if (tile < pr.ntx) {
+                batch_ghosts<double>(q, pr, b.Pin, b.Pout, tile, 0, TUBE_TX, 1, st == 0, t);
+                __threadfence_block();
+                __syncthreads();
+            }
+            // a last tile of one or two cells leaves the x-hi ghosts that it fills
+            // in the halo of the tile before it
+            if (st == 0 && short_last) tube_meet();
+            if (tile < pr.ntx) {
+                stage_tile<1, REC, RS, double, TUBE_TX, 1, 1, TUBE_TX, true>(q, b, tile, 0, 0, smem_raw);
+            }
+            tube_meet();
+        }
+        if (r.rk == 3) c ^= 1;  // an odd number of buffer swaps
+    }
+}
+
+bool tube_fits(int cells) { return cells <= TUBE_TX * TUBE_CLUSTER; }
+
+template <int REC, int RS>
+static cudaError_t launch_tube_t(const TubeRun& r, const BatchProb& pr, const StageParams& q, cudaStream_t s) {
+    auto kern = k_tube<REC, RS>;
+    constexpr size_t smem = TileGeom<1, TUBE_TX, 1, 1>::smem_bytes<double>();
+    static int widest[64] = {0};  // largest cluster per device; racing writers store the same value
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& wide = widest[dev & 63];
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(TUBE_TX);
+    cfg.dynamicSmemBytes = smem;
+    if (!wide) {
+        int fit = 0;
+        at.val.clusterDim.x = TUBE_CLUSTER;
+        cfg.gridDim = dim3(TUBE_CLUSTER);
+        const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0;
+        if (!ok) cudaGetLastError();
+        wide = ok ? TUBE_CLUSTER : 8;
+    }
+    int c = 1;
+    while (c < pr.ntx) c *= 2;
+    if (c > wide) return cudaErrorNotSupported;  // the caller takes the separate kernels
+    at.val.clusterDim.x = c;
+    cfg.gridDim = dim3(c);
+    return cudaLaunchKernelEx(&cfg, kern, r, pr, q);
+}
+
+cudaError_t launch_tube(int rec, int rs, const TubeRun& r, const int* bc_kind, const double (*bc_par)[16],
+                        const StageParams& p, cudaStream_t s) {
+    BatchProb pr{};
+    pr.dims = 1;
+    pr.n0 = p.n[0];
+    pr.n1 = 1;
+    pr.vs = p.vs;
+    pr.ntx = (p.n[0] - 2 * NG + TUBE_TX - 1) / TUBE_TX;
+    pr.nty = 1;
+    for (int f = 0; f < 2; ++f) {
+        pr.bc_kind[f] = bc_kind[f];
+        for (int k = 0; k < 8; ++k) pr.bc_par[f][k] = bc_par[f][k];
+    }
+#define VB_CASE(RC, RSC) \
+    if (rec == RC && rs == RSC) return launch_tube_t<RC, RSC>(r, pr, p, s);
+    VB_CASE(REC_MINMOD, RS_HLL)
+    VB_CASE(REC_MINMOD, RS_HLLC)
+    VB_CASE(REC_PPM, RS_HLL)
+    VB_CASE(REC_PPM, RS_HLLC)
+    VB_CASE(REC_WENOZ, RS_HLL)
+    VB_CASE(REC_WENOZ, RS_HLLC)
+#undef VB_CASE
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace vb
