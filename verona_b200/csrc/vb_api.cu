@@ -538,11 +538,15 @@ template <typename R> static int bc_fill(vb_handle h, R* P, cudaStream_t s) {
         VB_CUDA(h, launch_bc_decay<R>(g, P, face, (int)par[0], par[3], s));
         h->launches += 1;
     }
-    static const int order[6] = {2, 3, 4, 5, 0, 1};
-    for (int oi = 0; oi < 6; ++oi) {
-        int face = order[oi];
-        if (face / 2 >= h->dims || h->bc_kind[face] == VB_BC_FIXED) continue;
-        VB_CUDA(h, launch_bc_face<R>(g, P, face, h->bc_kind[face], h->bc_par[face], s));
+    BCFaces bc{};
+    bool any = false;
+    for (int face = 0; face < 2 * h->dims; ++face) {
+        bc.kind[face] = h->bc_kind[face];
+        for (int k = 0; k < 8; ++k) bc.par[face][k] = h->bc_par[face][k];
+        any = any || h->bc_kind[face] != VB_BC_FIXED;
+    }
+    if (any) {
+        VB_CUDA(h, launch_bc_fill<R>(g, P, bc, s));
         h->launches += 1;
     }
     return VB_OK;
@@ -593,6 +597,12 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
     const bool contract = std::is_same<R, double>::value && h->tun.fp64_contract == 1;
     if (contract && vb_f64c_stage_params_size() != sizeof(StageParams))
         return fail(h, VB_ERR_STATE, "vb_step: FMA-contracted FP64 unit built from another StageParams");
+    // the stage's last kernel copies the ghost cells where it has CTAs for them:
+    // the split con2prim kernels, the gated learned form's deferred pass, the 1D / 2D box kernel
+    const bool learned = p.skip_c2p != 0;
+    const bool gated = learned && h->tun.learned_fused != 0 && p.c2p_fp32 && h->defer_idx;
+    const bool last_does_ghosts = learned ? gated : (h->dims < 3 || stage_split_c2p<R>(h->dims, p));
+    p.ghosts = last_does_ghosts && !learned ? ghost_ctas(g, 128) : 0;
     auto stage = [&](const R* Pin, R* Pout, const double* Us, double* Uo, double dts, double a, double b) -> int {
         for (int d = 0; d < 3; ++d) p.dtdx[d] = d < h->dims ? dts / h->dx[d] : 0.0;
         p.tmap_in = p.tmap_row = nullptr;
@@ -617,6 +627,7 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
             StageParams q = p;
             q.skip_c2p = 1;
             q.want_div = 0;
+            q.ghosts = 0;
             if (contract)
                 VB_CUDA(h, vb_f64c_launch_stage(h->dims, h->opt.recon, h->opt.riemann, &q, &bufs, s, &nk));
             else
@@ -648,6 +659,7 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
                     q.defer_w0 = h->w_guess;
                     VB_CUDA(h, cudaMemsetAsync(h->defer_n, 0, sizeof(unsigned int), s));
                     VB_CUDA(h, launch_c2p_learned<R>(h->mlp_blob, q, bufs, h->tc_err, s));
+                    q.ghosts = ghost_ctas(g, 256);
                     VB_CUDA(h, launch_c2p_deferred<R>(q, bufs, s));
                     h->launches += 2;
                 } else {
@@ -662,8 +674,8 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
             }
         }
         if (h->prof) VB_CUDA(h, cudaEventRecord(e1, s));
-        VB_CUDA(h, launch_ghost_limit<R>(g, Pin, Pout, h->opt.floor_, s));
-        h->launches += nk + 1;
+        if (!last_does_ghosts) VB_CUDA(h, launch_ghost_limit<R>(g, Pin, Pout, h->opt.floor_, s));
+        h->launches += nk + (last_does_ghosts ? 0 : 1);
         h->stage_launches += 1;
         return VB_OK;
     };

@@ -43,7 +43,7 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // Ghost layers read by one tile: x-ghosts of its rows on an x edge, y-ghosts
 // of its columns on a y edge. At the first stage of a step (first) they are
 // filled as the single-grid solver fills them at the start of the step
-// (vb_set_boundary kinds, launch_bc_face / launch_bc_decay): OUTFLOW copies
+// (vb_set_boundary kinds, launch_bc_fill / launch_bc_decay): OUTFLOW copies
 // the first interior cell, NOZZLE holds the inflow state inside the radius
 // (cells measured from the centre along the face) and copies outside it,
 // FIXED keeps the loaded ghosts and multiplies the decaying variable by its

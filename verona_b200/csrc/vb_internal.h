@@ -49,6 +49,8 @@ struct StageParams {
     int div_in_pout;     // 1: the stencil kernel left the FP32 divergence in Pout; the
                          //    con2prim kernel forms Uo = rk_a U0 + rk_b (Us - div) itself
     int want_div;        // 1: the caller's con2prim kernel (skip_c2p) accepts div_in_pout
+    int ghosts;          // > 0: so many more CTAs of the stage's last kernel (con2prim, or the fused box
+                         //    kernel's extra column) copy and floor the ghost cells, Pin -> Pout
     int c2p_rescue;      // 1: 1D / 2D cells whose reference Newton diverges are solved by the
                          //    bracketed W Newton (batched problems); 0: kept and counted as failures
     const void* tmap_row; // host CUtensorMap of Pin by rows (encode_stage_row_tmap), for the TMA form of
@@ -97,12 +99,18 @@ struct InitIC {
 };
 template <typename R>
 cudaError_t launch_init_prims(const Grid& g, const InitIC& ic, R* P, double* U0, double gamma, cudaStream_t s);
+// CTAs of NT threads for StageParams::ghosts
+int ghost_ctas(const Grid& g, int nt);
 // ghost cells of Pout = limit(ghost cells of Pin)
 template <typename R>
 cudaError_t launch_ghost_limit(const Grid& g, const R* Pin, R* Pout, double floor_, cudaStream_t s);
-// boundary fill of one face (kind: 0 outflow, 2 nozzle); decay of a FIXED face
-template <typename R>
-cudaError_t launch_bc_face(const Grid& g, R* P, int face, int kind, const double* par, cudaStream_t s);
+// boundary fill of every face (kind: 0 outflow, 1 fixed, 2 nozzle with par {radius, c1,
+// c2, rho, u, u1, u2, u3}); decay of a FIXED face
+struct BCFaces {
+    int kind[6];
+    double par[6][8];
+};
+template <typename R> cudaError_t launch_bc_fill(const Grid& g, R* P, const BCFaces& bc, cudaStream_t s);
 template <typename R>
 cudaError_t launch_bc_decay(const Grid& g, R* P, int face, int var, double factor, cudaStream_t s);
 // per-block maxima of the CFL signal speed into partial[], then one block reduces them to out

@@ -45,6 +45,7 @@
 #include "vb_con2prim.cuh"
 #include "vb_index.cuh"
 #include "vb_internal.h"
+#include "vb_stage.cuh"
 #include "vb_tc.cuh"
 
 namespace vb {
@@ -1016,6 +1017,11 @@ template cudaError_t launch_c2p_learned<double>(const void*, const StageParams&,
 template <typename R>
 __global__ void __launch_bounds__(256) k_c2p_deferred(StageParams p, StageBufs<R> b) {
     const int N0 = p.n[0] - 2 * NG, N1 = p.n[1] - 2 * NG, N2 = p.n[2] - 2 * NG;
+    const int ctas = (int)gridDim.x - p.ghosts;  // the last p.ghosts CTAs do the ghost cells
+    if ((int)blockIdx.x >= ctas) {
+        ghost_copy<R, 5>(p.n, p.sy, p.sz, p.vs, b.Pin, b.Pout, R(p.floor_), blockIdx.x - ctas, p.ghosts);
+        return;
+    }
     const unsigned long long cap = (unsigned long long)N0 * N1 * N2;
     const unsigned long long n = std::min<unsigned long long>(*p.defer_n, cap);
     CellMap cm;  // interior cells < 2^32 (launch_c2p_deferred)
@@ -1023,7 +1029,7 @@ __global__ void __launch_bounds__(256) k_c2p_deferred(StageParams p, StageBufs<R
     const long long vs = p.vs;
     unsigned long long n_fail = 0, n_fb = 0, n_it = 0, n_cells = 0;
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
+         i += (unsigned long long)ctas * blockDim.x) {
         const unsigned e = p.defer_idx[i];
         if ((unsigned long long)e >= cap) {
             if (p.counters) atomicAdd(p.counters + CNT_BAD_INDEX, 1ULL);
@@ -1074,7 +1080,7 @@ template <typename R> cudaError_t launch_c2p_deferred(const StageParams& p, cons
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int nb = (int)std::max<long long>(1, std::min<long long>((cells + 255) / 256, 8LL * std::max(1, sms)));
-    k_c2p_deferred<R><<<nb, 256, 0, s>>>(p, b);
+    k_c2p_deferred<R><<<nb + p.ghosts, 256, 0, s>>>(p, b);
     return cudaGetLastError();
 }
 template cudaError_t launch_c2p_deferred<float>(const StageParams&, const StageBufs<float>&, cudaStream_t);

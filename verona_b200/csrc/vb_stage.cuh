@@ -79,6 +79,51 @@ template <typename R, int TX, int TY> bool encode_tile2_tmap(void* out, const R*
     return encode_tmap(out, P, (int)sizeof(R), 3, dim, stride, box);
 }
 
+// ---- ghost cells ---------------------------------------------------------------
+// The ghost region is covered by disjoint slabs: x-lo/x-hi over all (j,k);
+// y-lo/y-hi over interior i and all k; z-lo/z-hi over interior (i,j). Slab s is
+// side s % 2 of axis s / 2; a slab has fewer than 2^32 cells (the padded grid of
+// a handle that fits this GPU does).
+template <int DIM> __host__ __device__ __forceinline__ uint32_t ghost_slab_size(const int* n, int axis) {
+    if (axis >= DIM) return 0;
+    const uint32_t e0 = axis == 0 ? NG : n[0] - 2 * NG, e1 = DIM < 2 ? 1 : (axis == 1 ? NG : (axis == 2 ? n[1] - 2 * NG : n[1])),
+                   e2 = DIM < 3 ? 1 : (axis == 2 ? NG : n[2]);
+    return e0 * e1 * e2;
+}
+// cell e of a slab -> padded (i, j, k)
+template <int DIM> __device__ __forceinline__ void ghost_slab_cell(const int* n, int slab, uint32_t e, int* x) {
+    const int a = slab >> 1, side = slab & 1;
+    const uint32_t e0 = a == 0 ? NG : n[0] - 2 * NG;
+    const uint32_t e1 = DIM < 2 ? 1 : (a == 1 ? NG : (a == 2 ? n[1] - 2 * NG : n[1]));
+    const uint32_t row = e / e0, pl = DIM < 3 ? 0 : row / e1;
+    x[0] = (int)(e - row * e0) + (a == 0 ? (side ? n[0] - NG : 0) : NG);
+    x[1] = DIM < 2 ? 0 : (int)(row - pl * e1) + (a == 1 ? (side ? n[1] - NG : 0) : (a == 2 ? NG : 0));
+    x[2] = DIM < 3 ? 0 : (int)pl + (a == 2 ? (side ? n[2] - NG : 0) : 0);
+}
+// ghost cells of Pout = limit(ghost cells of Pin) (function_Limit,
+// src/3dim/algos.jl:5-12), by CTA `cta` of `ctas`
+template <typename R, int NV>
+__device__ __forceinline__ void ghost_copy(const int* n, long long sy, long long sz, long long vs, const R* Pin, R* Pout,
+                                           R fl, uint32_t cta, uint32_t ctas) {
+    constexpr int DIM = NV - 2;
+#pragma unroll 1
+    for (int slab = 0; slab < 2 * DIM; ++slab) {
+        const uint32_t tot = ghost_slab_size<DIM>(n, slab >> 1);
+        for (uint32_t e = cta * blockDim.x + threadIdx.x; e < tot; e += ctas * blockDim.x) {
+            int x[3];
+            ghost_slab_cell<DIM>(n, slab, e, x);
+            const long long c = x[0] + sy * x[1] + sz * x[2];
+            R q[NV];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) q[v] = Pin[v * vs + c];
+            q[0] = jmax(q[0], fl);
+            q[1] = jmax(q[1], fl);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) Pout[v * vs + c] = q[v];
+        }
+    }
+}
+
 __device__ __forceinline__ void count_add(unsigned long long* c, int which, unsigned long long v) {
     if (c && v) atomicAdd(c + which, v);
 }
@@ -452,6 +497,10 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs
 template <int DIM, int REC, int RS, typename R, int TX, int TY, int TZ, int NT, bool TMA>
 __global__ void __launch_bounds__(NT) k_stage(StageParams p, StageBufs<R> b, const __grid_constant__ CUtensorMap tm) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (DIM < 3 && p.ghosts && blockIdx.x == gridDim.x - 1) {  // the extra column of CTAs
+        ghost_copy<R, 2 + DIM>(p.n, p.sy, p.sz, p.vs, b.Pin, b.Pout, R(p.floor_), blockIdx.y, gridDim.y);
+        return;
+    }
     stage_tile<DIM, REC, RS, R, TX, TY, TZ, NT, false, TMA>(p, b, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z,
                                                             smem_raw, &tm);
 }
@@ -477,7 +526,7 @@ cudaError_t launch_stage_tt(const StageParams& p, const StageBufs<R>& b, cudaStr
         if (e != cudaSuccess) return e;
         attr_set |= 1ULL << (dev & 63);
     }
-    dim3 grid((p.n[0] - 2 * NG + C::TX - 1) / C::TX, DIM > 1 ? (p.n[1] - 2 * NG + C::TY - 1) / C::TY : 1,
+    dim3 grid((p.n[0] - 2 * NG + C::TX - 1) / C::TX + (DIM < 3 && p.ghosts ? 1 : 0), DIM > 1 ? (p.n[1] - 2 * NG + C::TY - 1) / C::TY : 1,
               DIM > 2 ? (p.n[2] - 2 * NG + C::TZ - 1) / C::TZ : 1);
     CUtensorMap tm;
     if (TMA)
@@ -535,6 +584,7 @@ cudaError_t launch_stage(int dims, int rec, int rs, const StageParams& p, const 
         // split: the box kernel writes U only, then k_c2p_2d
         StageParams q = p;
         q.skip_c2p = 1;
+        q.ghosts = 0;
         const cudaError_t e = dispatch_stage_dim<2, R>(rec, rs, q, b, s);
         if (e != cudaSuccess) return e;
         *kernels = 2;
@@ -766,112 +816,84 @@ cudaError_t launch_store_prims(const Grid& g, const R* P, double* Pa, cudaStream
     return cudaGetLastError();
 }
 
-// ---- ghost cells -------------------------------------------------------------
-// The ghost region is covered by disjoint slabs: x-lo/x-hi over all (j,k);
-// y-lo/y-hi over interior i and all k; z-lo/z-hi over interior (i,j).
-__device__ __forceinline__ bool ghost_slab_cell(const Grid& g, int slab, long long e, int& i, int& j, int& k) {
-    const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
-    const int a = slab / 2, side = slab % 2;
-    int ext[3];
-    int lo[3];
-    if (a == 0) {
-        ext[0] = NG; ext[1] = n1; ext[2] = n2;
-        lo[0] = side ? n0 - NG : 0; lo[1] = 0; lo[2] = 0;
-    } else if (a == 1) {
-        ext[0] = n0 - 2 * NG; ext[1] = NG; ext[2] = n2;
-        lo[0] = NG; lo[1] = side ? n1 - NG : 0; lo[2] = 0;
-    } else {
-        ext[0] = n0 - 2 * NG; ext[1] = n1 - 2 * NG; ext[2] = NG;
-        lo[0] = NG; lo[1] = NG; lo[2] = side ? n2 - NG : 0;
-    }
-    long long tot = (long long)ext[0] * ext[1] * ext[2];
-    if (e >= tot) return false;
-    i = lo[0] + (int)(e % ext[0]);
-    j = lo[1] + (int)((e / ext[0]) % ext[1]);
-    k = lo[2] + (int)(e / ((long long)ext[0] * ext[1]));
-    return true;
-}
-
-template <typename R>
-__global__ void k_ghost_limit(Grid g, const R* __restrict__ Pin, R* __restrict__ Pout, double floor_) {
-    const int slab = blockIdx.y;
-    const R fl = R(floor_);
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;; e += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        if (!ghost_slab_cell(g, slab, e, i, j, k)) break;
-        long long c = i + g.sy * j + g.sz * k;
-        for (int v = 0; v < g.nv; ++v) {
-            R x = Pin[v * g.vs + c];
-            if (v < 2) x = jmax(x, fl);  // function_Limit, src/3dim/algos.jl:5-12
-            Pout[v * g.vs + c] = x;
-        }
-    }
+// ---- ghost cells: kernels of their own (ghost_slab_cell and ghost_copy above) ----
+template <typename R, int NV>
+__global__ void __launch_bounds__(256) k_ghost_limit(Grid g, const R* __restrict__ Pin, R* __restrict__ Pout, double floor_) {
+    ghost_copy<R, NV>(g.n, g.sy, g.sz, g.vs, Pin, Pout, R(floor_), blockIdx.x, gridDim.x);
 }
 
 template <typename R>
 cudaError_t launch_ghost_limit(const Grid& g, const R* Pin, R* Pout, double floor_, cudaStream_t s) {
-    long long maxslab = (long long)NG * g.n[1] * g.n[2];
-    if (g.dims > 1) maxslab = max(maxslab, (long long)NG * g.n[0] * g.n[2]);
-    if (g.dims > 2) maxslab = max(maxslab, (long long)NG * g.n[0] * g.n[1]);
-    dim3 grid(grid_for(maxslab, 256), 2 * g.dims);
-    k_ghost_limit<R><<<grid, 256, 0, s>>>(g, Pin, Pout, floor_);
+    const int nb = ghost_ctas(g, 256);
+    if (g.dims == 1) k_ghost_limit<R, 3><<<nb, 256, 0, s>>>(g, Pin, Pout, floor_);
+    else if (g.dims == 2) k_ghost_limit<R, 4><<<nb, 256, 0, s>>>(g, Pin, Pout, floor_);
+    else k_ghost_limit<R, 5><<<nb, 256, 0, s>>>(g, Pin, Pout, floor_);
     return cudaGetLastError();
 }
 
-// Boundary fill of one face, the on-device replacement of the reference's
-// host-side `fun_bound` broadcasts (examples/Jet3D/HARM_jet_breakout.jl:131-158):
-// OUTFLOW copies the first interior cell into the 3 ghost layers over the
-// full padded extent of the other axes; NOZZLE holds a fixed state inside a
-// radius (cells, from a centre in the face plane) and is OUTFLOW outside.
-// par: NOZZLE {radius, c1, c2, rho, u, u1, u2, u3}.
-struct BCPar {
-    double v[8];
-};
-
-template <typename R>
-__global__ void k_bc_face(Grid g, R* __restrict__ P, int face, int kind, BCPar par) {
-    const int a = face / 2, side = face % 2;
-    const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
-    int ext[3] = {n0, n1, n2};
-    ext[a] = NG;
-    long long tot = (long long)ext[0] * ext[1] * ext[2];
-    int b1 = (a + 1) % 3, b2 = (a + 2) % 3;
-    if (b1 > b2) {
-        int t = b1;
-        b1 = b2;
-        b2 = t;
-    }
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
-        int idx[3] = {(int)(e % ext[0]), (int)((e / ext[0]) % ext[1]), (int)(e / ((long long)ext[0] * ext[1]))};
-        if (side) idx[a] += g.n[a] - NG;
-        long long c = idx[0] + g.sy * idx[1] + g.sz * idx[2];
-        bool inside = false;
-        if (kind == 2) {
-            double y1 = (b1 < g.dims) ? (idx[b1] - NG + 0.5) - par.v[1] : 0.0;
-            double y2 = (b2 < g.dims) ? (idx[b2] - NG + 0.5) - par.v[2] : 0.0;
-            inside = y1 * y1 + y2 * y2 < par.v[0] * par.v[0];
-        }
-        if (inside) {
-            P[c] = (R)par.v[3];
-            P[g.vs + c] = (R)par.v[4];
-            for (int m = 0; m < g.dims; ++m) P[(2 + m) * g.vs + c] = (R)par.v[5 + m];
-        } else {
-            int s[3] = {idx[0], idx[1], idx[2]};
-            s[a] = side ? g.n[a] - NG - 1 : NG;
-            long long cs = s[0] + g.sy * s[1] + g.sz * s[2];
-            for (int v = 0; v < g.nv; ++v) P[v * g.vs + c] = P[v * g.vs + cs];
+// Boundary fill of every face at the start of a step, the on-device replacement
+// of the reference's host-side `fun_bound` broadcasts
+// (examples/Jet3D/HARM_jet_breakout.jl:131-158). Face by face in the order y, z,
+// x, each over the full padded extent of the other axes, OUTFLOW copies the first
+// interior cell into the 3 ghost layers, NOZZLE holds a fixed state inside a
+// radius (cells, from a centre in the face plane) and is OUTFLOW outside, FIXED
+// leaves the ghosts alone. Here one launch does all faces: each ghost cell follows
+// that order backwards to the cell its value ends up coming from, which no face
+// writes (an interior cell, or a ghost cell of FIXED faces only).
+template <typename R, int DIM>
+__global__ void __launch_bounds__(256) k_bc_fill(Grid g, R* __restrict__ P, BCFaces bc) {
+    constexpr int NV = 2 + DIM;
+    const int slabs = 2 * DIM;
+    const uint32_t tot0 = ghost_slab_size<DIM>(g.n, 0), tot1 = ghost_slab_size<DIM>(g.n, 1),
+                   tot2 = ghost_slab_size<DIM>(g.n, 2);
+    for (int slab = 0; slab < slabs; ++slab) {
+        const uint32_t tot = slab < 2 ? tot0 : (slab < 4 ? tot1 : tot2);
+        for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {
+            int x[3];
+            ghost_slab_cell<DIM>(g.n, slab, e, x);
+            const long long c = x[0] + g.sy * x[1] + g.sz * x[2];
+            bool moved = false;
+            int inflow = -1;  // the face whose nozzle holds the value
+#pragma unroll
+            for (int o = 0; o < 3; ++o) {
+                const int a = o == 0 ? 0 : (o == 1 ? 2 : 1);  // x was filled last, then z, then y
+                if (a >= DIM || inflow >= 0) continue;
+                const int side = x[a] < NG ? 0 : (x[a] >= g.n[a] - NG ? 1 : -1);
+                if (side < 0) continue;
+                const int f = 2 * a + side;
+                if (bc.kind[f] == 1) continue;
+                if (bc.kind[f] == 2) {
+                    const int b1 = a == 0 ? 1 : 0, b2 = a == 2 ? 1 : 2;
+                    const double y1 = b1 < DIM ? (x[b1] - NG + 0.5) - bc.par[f][1] : 0.0;
+                    const double y2 = b2 < DIM ? (x[b2] - NG + 0.5) - bc.par[f][2] : 0.0;
+                    if (y1 * y1 + y2 * y2 < bc.par[f][0] * bc.par[f][0]) {
+                        inflow = f;
+                        continue;
+                    }
+                }
+                x[a] = side ? g.n[a] - NG - 1 : NG;
+                moved = true;
+            }
+            if (inflow >= 0) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) P[v * g.vs + c] = (R)bc.par[inflow][3 + v];
+            } else if (moved) {
+                const long long cs = x[0] + g.sy * x[1] + g.sz * x[2];
+                R q[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) q[v] = P[v * g.vs + cs];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) P[v * g.vs + c] = q[v];
+            }
         }
     }
 }
 
-template <typename R>
-cudaError_t launch_bc_face(const Grid& g, R* P, int face, int kind, const double* par, cudaStream_t s) {
-    BCPar bp;
-    for (int i = 0; i < 8; ++i) bp.v[i] = par ? par[i] : 0.0;
-    int a = face / 2;
-    long long tot = (long long)g.n[0] * g.n[1] * g.n[2] / g.n[a] * NG;
-    k_bc_face<R><<<grid_for(tot, 256), 256, 0, s>>>(g, P, face, kind, bp);
+template <typename R> cudaError_t launch_bc_fill(const Grid& g, R* P, const BCFaces& bc, cudaStream_t s) {
+    const int nb = ghost_ctas(g, 256);
+    if (g.dims == 1) k_bc_fill<R, 1><<<nb, 256, 0, s>>>(g, P, bc);
+    else if (g.dims == 2) k_bc_fill<R, 2><<<nb, 256, 0, s>>>(g, P, bc);
+    else k_bc_fill<R, 3><<<nb, 256, 0, s>>>(g, P, bc);
     return cudaGetLastError();
 }
 
@@ -975,7 +997,7 @@ cudaError_t launch_max_speed(const Grid& g, const R* P, double gamma, double* pa
     template cudaError_t launch_init_prims<R>(const Grid&, const InitIC&, R*, double*, double, cudaStream_t); \
     template cudaError_t launch_pack_interior<R>(const Grid&, const R*, double*, unsigned long long*, cudaStream_t); \
     template cudaError_t launch_ghost_limit<R>(const Grid&, const R*, R*, double, cudaStream_t);      \
-    template cudaError_t launch_bc_face<R>(const Grid&, R*, int, int, const double*, cudaStream_t);  \
+    template cudaError_t launch_bc_fill<R>(const Grid&, R*, const BCFaces&, cudaStream_t);           \
     template cudaError_t launch_bc_decay<R>(const Grid&, R*, int, int, double, cudaStream_t);        \
     template cudaError_t launch_max_speed<R>(const Grid&, const R*, double, double*, int, double*,   \
                                              cudaStream_t);                                          \

@@ -128,6 +128,17 @@ cudaError_t launch_point_c2p_gated(double g, const double* U, const float* W0, d
     return cudaGetLastError();
 }
 
+int ghost_ctas(const Grid& g, int nt) {
+    long long cells = 1, inner = 1;
+    for (int a = 0; a < g.dims; ++a) {
+        cells *= g.n[a];
+        inner *= g.n[a] - 2 * NG;
+    }
+    // about two cells a thread, at most four CTAs per SM
+    const long long b = (cells - inner + 2 * nt - 1) / (2 * nt);
+    return (int)std::max(1LL, std::min(b, 4LL * sm_count()));
+}
+
 int max_speed_blocks(const Grid& g) {
     (void)g;
     return 148 * 4;

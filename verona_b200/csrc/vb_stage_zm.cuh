@@ -391,11 +391,16 @@ __global__ void __launch_bounds__(C2pCfg<MODE>::NT, C2pCfg<MODE>::MINB) k_c2p(St
     constexpr int NV = 5;
     const int N0 = p.n[0] - 2 * NG, N1 = p.n[1] - 2 * NG, N2 = p.n[2] - 2 * NG;
     const long long tot = (long long)N0 * N1 * N2;  // < 2^32 (launch_c2p)
+    const int ctas = (int)gridDim.x - p.ghosts;  // the last p.ghosts CTAs do the ghost cells
+    if ((int)blockIdx.x >= ctas) {
+        ghost_copy<R, NV>(p.n, p.sy, p.sz, p.vs, b.Pin, b.Pout, R(p.floor_), blockIdx.x - ctas, p.ghosts);
+        return;
+    }
     CellMap cm;
     cm.init(N0, N1, p.sy, p.sz, NG);
     unsigned long long n_fail = 0, n_fb = 0, n_it = 0, n_cells = 0, n_64 = 0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
+         e += (long long)ctas * blockDim.x) {
         const long long c = cm.padded((uint32_t)e);
         double U[NV], P[NV];
         const bool need_p = !(p.c2p_mode == C2P_GUESS_W && p.w_guess);
@@ -447,11 +452,16 @@ __global__ void __launch_bounds__(C2p2dCfg<MODE>::NT, C2p2dCfg<MODE>::MINB) k_c2
     constexpr int NV = 4;
     const int N0 = p.n[0] - 2 * NG, N1 = p.n[1] - 2 * NG;
     const long long tot = (long long)N0 * N1;  // < 2^32 (launch_c2p)
+    const int ctas = (int)gridDim.x - p.ghosts;  // the last p.ghosts CTAs do the ghost cells
+    if ((int)blockIdx.x >= ctas) {
+        ghost_copy<R, NV>(p.n, p.sy, p.sz, p.vs, b.Pin, b.Pout, R(p.floor_), blockIdx.x - ctas, p.ghosts);
+        return;
+    }
     CellMap cm;
     cm.init(N0, N1, p.sy, p.sz, NG);
     unsigned long long n_fail = 0, n_fb = 0, n_it = 0, n_cells = 0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
-         e += (long long)gridDim.x * blockDim.x) {
+         e += (long long)ctas * blockDim.x) {
         // interior cell (i, j) -> (i + NG) + sy (j + NG); the z index stays 0
         const uint32_t j = cm.dx.div((uint32_t)e), i = (uint32_t)e - j * cm.n0;
         const long long c = (long long)(i + NG) + p.sy * (long long)(j + NG);
@@ -514,17 +524,17 @@ template <typename R> cudaError_t launch_c2p(const StageParams& p, const StageBu
         const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG);
         if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
         if (p.c2p_mode == C2P_GUESS_W)
-            k_c2p_2d<R, 2><<<grid_for(cells, C2p2dCfg<2>::NT), C2p2dCfg<2>::NT, 0, s>>>(p, b);
+            k_c2p_2d<R, 2><<<grid_for(cells, C2p2dCfg<2>::NT) + p.ghosts, C2p2dCfg<2>::NT, 0, s>>>(p, b);
         else
-            k_c2p_2d<R, 1><<<grid_for(cells, C2p2dCfg<1>::NT), C2p2dCfg<1>::NT, 0, s>>>(p, b);
+            k_c2p_2d<R, 1><<<grid_for(cells, C2p2dCfg<1>::NT) + p.ghosts, C2p2dCfg<1>::NT, 0, s>>>(p, b);
         return cudaGetLastError();
     }
     const long long cells = (long long)(p.n[0] - 2 * NG) * (p.n[1] - 2 * NG) * (p.n[2] - 2 * NG);
     if ((unsigned long long)cells > MAX_CELLS_U32) return cudaErrorInvalidValue;
     if (p.c2p_mode == C2P_GUESS_W)
-        k_c2p<R, 2><<<grid_for(cells, C2pCfg<2>::NT), C2pCfg<2>::NT, 0, s>>>(p, b);
+        k_c2p<R, 2><<<grid_for(cells, C2pCfg<2>::NT) + p.ghosts, C2pCfg<2>::NT, 0, s>>>(p, b);
     else
-        k_c2p<R, 1><<<grid_for(cells, C2pCfg<1>::NT), C2pCfg<1>::NT, 0, s>>>(p, b);
+        k_c2p<R, 1><<<grid_for(cells, C2pCfg<1>::NT) + p.ghosts, C2pCfg<1>::NT, 0, s>>>(p, b);
     return cudaGetLastError();
 }
 
