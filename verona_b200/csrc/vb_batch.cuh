@@ -18,8 +18,8 @@
 //     too small by vb_batch_set_wait_limit) counts CNT_TIMEOUT and stops the
 //     CTA. The tiles that depend on the stopped one then run out in turn, so
 //     the launch ends in bounded time; vb_batch_check reports it.
-//   * The tile itself is the box-tile stage body (stage_tile, vb_stage.cuh)
-//     with loads through L2, so data written earlier in the launch by other
+//   * The tile itself is the box-tile stage body (stage_tile, vb_stage.cuh; FP32
+//     bulk on packed pairs, vb_tile_pk.cuh) with loads through L2, so data written earlier in the launch by other
 //     SMs is seen.
 //   * Ghost cells follow the single-grid solver exactly: at the first stage of
 //     a step a tile on a domain edge copies the first interior cell into the
@@ -28,9 +28,11 @@
 //     stage output; later stages copy the floored ghosts of their input.
 #pragma once
 #include "vb_ns.h"
+#include <algorithm>
 #include <type_traits>
 #include "vb_batch.h"
 #include "vb_stage.cuh"
+#include "vb_tile_pk.cuh"
 
 namespace VB_NS {
 
@@ -112,11 +114,36 @@ __device__ __forceinline__ void batch_ghosts(const StageParams& q, const BatchPr
     }
 }
 
+// tile shapes of the kernel variants the autotuner chooses among, and the CTAs per
+// SM that the registers are held to
+template <typename R> struct BatchVariants;
+template <> struct BatchVariants<float> {
+    static constexpr int N = 4, MINB = 4;
+    static constexpr int TX2[N] = {32, 32, 64, 16}, TY2[N] = {8, 16, 4, 16}, L1[N] = {256, 512, 128, 256};
+};
+template <> struct BatchVariants<double> {
+    static constexpr int N = 2, MINB = 1;
+    static constexpr int TX2[N] = {32, 16}, TY2[N] = {8, 8}, L1[N] = {256, 128};
+};
+
+// one tile of a stage: FP32 bulk on packed pairs, FP64 the box tile
+template <int DIM, int REC, int RS, typename R, int TX, int TY>
+__device__ __forceinline__ void batch_tile(const StageParams& q, const StageBufs<R>& b, int bx, int by,
+                                           unsigned char* smem_raw) {
+    if constexpr (sizeof(R) == 4)
+        stage_tile_pk<DIM, REC, RS, TX, TY, batch_nt<R>()>(q, b, bx, by, smem_raw);
+    else
+        stage_tile<DIM, REC, RS, R, TX, TY, 1, batch_nt<R>(), true>(q, b, bx, by, 0, smem_raw);
+}
+
 template <typename R, int RS, int TX2, int TY2, int L1>
-__global__ void __launch_bounds__(BATCH_NT) k_batch(BatchLaunch<R> a) {
+__global__ void __launch_bounds__(batch_nt<R>(), BatchVariants<R>::MINB) k_batch(BatchLaunch<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ long long s_ticket;
     __shared__ int s_ok;
+    // this ticket's stage, in shared memory: as locals its ~50 words took the tiles' registers
+    __shared__ StageParams s_q;
+    __shared__ StageBufs<R> s_b;
     for (;;) {
         if (threadIdx.x == 0) s_ticket = (long long)atomicAdd(a.next, 1ULL);
         __syncthreads();
@@ -149,48 +176,55 @@ __global__ void __launch_bounds__(BATCH_NT) k_batch(BatchLaunch<R> a) {
         R* Pn = (c ? a.P0 : a.P1) + pr.offP;
         double* U0 = a.U0 + pr.offU;
         double* U1 = a.U1 + pr.offU;
-        StageParams q{};
-        q.n[0] = pr.n0;
-        q.n[1] = pr.n1;
-        q.n[2] = 1;
-        q.sy = pr.n0;
-        q.sz = (long long)pr.n0 * pr.n1;
-        q.vs = pr.vs;
-        q.gamma = a.gamma;
-        q.floor_ = a.floor_;
-        q.tol = a.tol;
-        q.n_iter = a.n_iter;
-        q.stats = a.stats;
-        // FP64: the reference con2prim (parity with the single-grid solver);
-        // FP32 bulk: the W Newton from the input state first (cheaper, no LU)
-        q.c2p_mode = std::is_same<R, float>::value ? C2P_GUESS_W : C2P_REFERENCE;
-        q.c2p_rescue = 1;
-        q.w_rtol = 1e-12;
-        q.w_max_newton = 8;
-        q.counters = a.counters;
-        const bool half = a.rk == 2 && st == 0;
-        q.dtdx[0] = half ? pr.dtdx[1][0] : pr.dtdx[0][0];
-        q.dtdx[1] = pr.dims > 1 ? (half ? pr.dtdx[1][1] : pr.dtdx[0][1]) : 0.0;
-        q.dtdx[2] = 0.0;
-        StageBufs<R> b;
-        if (a.rk == 3) {
-            // SSP-RK3: U1 = U - dt L(P); U2 = 3/4 U + 1/4 (U1 - dt L(P1)); U = 1/3 U + 2/3 (U2 - dt L(P2))
-            q.rk_a = st == 0 ? 0.0 : (st == 1 ? 0.75 : 1.0 / 3.0);
-            q.rk_b = st == 0 ? 1.0 : (st == 1 ? 0.25 : 2.0 / 3.0);
-            b.Pin = (st & 1) ? Pn : Pc;
-            b.Pout = (st & 1) ? Pc : Pn;
-            b.Us = st == 0 ? U0 : U1;
-            b.Uo = st == 2 ? U0 : U1;
-        } else {
-            // midpoint RK2: Uhalf = U - dt/2 L(P); U = U - dt L(Phalf)
-            q.rk_a = 0.0;
-            q.rk_b = 1.0;
-            b.Pin = st ? Pn : Pc;
-            b.Pout = st ? Pc : Pn;
-            b.Us = U0;
-            b.Uo = st ? U0 : U1;
+        if (threadIdx.x == 0) {
+            StageParams q{};
+            q.n[0] = pr.n0;
+            q.n[1] = pr.n1;
+            q.n[2] = 1;
+            q.sy = pr.n0;
+            q.sz = (long long)pr.n0 * pr.n1;
+            q.vs = pr.vs;
+            q.gamma = a.gamma;
+            q.floor_ = a.floor_;
+            q.tol = a.tol;
+            q.n_iter = a.n_iter;
+            q.stats = a.stats;
+            // FP64: the reference con2prim (parity with the single-grid solver);
+            // FP32 bulk: the W Newton from the input state first (cheaper, no LU)
+            q.c2p_mode = std::is_same<R, float>::value ? C2P_GUESS_W : C2P_REFERENCE;
+            q.c2p_rescue = 1;
+            q.w_rtol = 1e-12;
+            q.w_max_newton = 8;
+            q.counters = a.counters;
+            const bool half = a.rk == 2 && st == 0;
+            q.dtdx[0] = half ? pr.dtdx[1][0] : pr.dtdx[0][0];
+            q.dtdx[1] = pr.dims > 1 ? (half ? pr.dtdx[1][1] : pr.dtdx[0][1]) : 0.0;
+            q.dtdx[2] = 0.0;
+            StageBufs<R> b;
+            if (a.rk == 3) {
+                // SSP-RK3: U1 = U - dt L(P); U2 = 3/4 U + 1/4 (U1 - dt L(P1)); U = 1/3 U + 2/3 (U2 - dt L(P2))
+                q.rk_a = st == 0 ? 0.0 : (st == 1 ? 0.75 : 1.0 / 3.0);
+                q.rk_b = st == 0 ? 1.0 : (st == 1 ? 0.25 : 2.0 / 3.0);
+                b.Pin = (st & 1) ? Pn : Pc;
+                b.Pout = (st & 1) ? Pc : Pn;
+                b.Us = st == 0 ? U0 : U1;
+                b.Uo = st == 2 ? U0 : U1;
+            } else {
+                // midpoint RK2: Uhalf = U - dt/2 L(P); U = U - dt L(Phalf)
+                q.rk_a = 0.0;
+                q.rk_b = 1.0;
+                b.Pin = st ? Pn : Pc;
+                b.Pout = st ? Pc : Pn;
+                b.Us = U0;
+                b.Uo = st ? U0 : U1;
+            }
+            b.U0 = U0;
+            s_q = q;
+            s_b = b;
         }
-        b.U0 = U0;
+        __syncthreads();
+        const StageParams& q = s_q;
+        const StageBufs<R>& b = s_b;
 
         const int TXc = pr.dims == 1 ? L1 : TX2, TYc = pr.dims == 1 ? 1 : TY2;
         // the problem's time at the start of this step: its time at the start
@@ -201,19 +235,13 @@ __global__ void __launch_bounds__(BATCH_NT) k_batch(BatchLaunch<R> a) {
         __threadfence_block();
         __syncthreads();
         if (pr.dims == 1) {
-            if (pr.rec == REC_MINMOD)
-                stage_tile<1, REC_MINMOD, RS, R, L1, 1, 1, BATCH_NT, true>(q, b, e.x, 0, 0, smem_raw);
-            else if (pr.rec == REC_PPM)
-                stage_tile<1, REC_PPM, RS, R, L1, 1, 1, BATCH_NT, true>(q, b, e.x, 0, 0, smem_raw);
-            else
-                stage_tile<1, REC_WENOZ, RS, R, L1, 1, 1, BATCH_NT, true>(q, b, e.x, 0, 0, smem_raw);
+            if (pr.rec == REC_MINMOD) batch_tile<1, REC_MINMOD, RS, R, L1, 1>(q, b, e.x, 0, smem_raw);
+            else if (pr.rec == REC_PPM) batch_tile<1, REC_PPM, RS, R, L1, 1>(q, b, e.x, 0, smem_raw);
+            else batch_tile<1, REC_WENOZ, RS, R, L1, 1>(q, b, e.x, 0, smem_raw);
         } else {
-            if (pr.rec == REC_MINMOD)
-                stage_tile<2, REC_MINMOD, RS, R, TX2, TY2, 1, BATCH_NT, true>(q, b, e.x, e.y, 0, smem_raw);
-            else if (pr.rec == REC_PPM)
-                stage_tile<2, REC_PPM, RS, R, TX2, TY2, 1, BATCH_NT, true>(q, b, e.x, e.y, 0, smem_raw);
-            else
-                stage_tile<2, REC_WENOZ, RS, R, TX2, TY2, 1, BATCH_NT, true>(q, b, e.x, e.y, 0, smem_raw);
+            if (pr.rec == REC_MINMOD) batch_tile<2, REC_MINMOD, RS, R, TX2, TY2>(q, b, e.x, e.y, smem_raw);
+            else if (pr.rec == REC_PPM) batch_tile<2, REC_PPM, RS, R, TX2, TY2>(q, b, e.x, e.y, smem_raw);
+            else batch_tile<2, REC_WENOZ, RS, R, TX2, TY2>(q, b, e.x, e.y, smem_raw);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -223,21 +251,11 @@ __global__ void __launch_bounds__(BATCH_NT) k_batch(BatchLaunch<R> a) {
     }
 }
 
-// tile shapes of the kernel variants the autotuner chooses among
-template <typename R> struct BatchVariants;
-template <> struct BatchVariants<float> {
-    static constexpr int N = 4;
-    static constexpr int TX2[N] = {32, 32, 64, 16}, TY2[N] = {8, 16, 4, 16}, L1[N] = {256, 512, 128, 256};
-};
-template <> struct BatchVariants<double> {
-    static constexpr int N = 2;
-    static constexpr int TX2[N] = {32, 16}, TY2[N] = {8, 8}, L1[N] = {256, 128};
-};
-
 template <typename R, int TX2, int TY2, int L1> constexpr size_t batch_smem() {
-    return TileGeom<2, TX2, TY2, 1>::template smem_bytes<R>() > TileGeom<1, L1, 1, 1>::template smem_bytes<R>()
-               ? TileGeom<2, TX2, TY2, 1>::template smem_bytes<R>()
-               : TileGeom<1, L1, 1, 1>::template smem_bytes<R>();
+    if constexpr (sizeof(R) == 4)
+        return std::max(PkTile<2, TX2, TY2, batch_nt<R>()>::smem_bytes(), PkTile<1, L1, 1, batch_nt<R>()>::smem_bytes());
+    else
+        return std::max(TileGeom<2, TX2, TY2, 1>::template smem_bytes<R>(), TileGeom<1, L1, 1, 1>::template smem_bytes<R>());
 }
 
 // launch = false: set the kernel attributes and compute the grid only (before
@@ -259,7 +277,7 @@ cudaError_t batch_launch_t(const BatchLaunch<R>& a, int ctas_per_sm, cudaStream_
     int nsm = 0, maxb = 0;
     cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, kern, BATCH_NT, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, kern, batch_nt<R>(), smem);
     if (e != cudaSuccess) return e;
     if (maxb < 1) return cudaErrorInvalidConfiguration;
     const int per = ctas_per_sm > 0 ? std::min(ctas_per_sm, maxb) : maxb;
@@ -267,7 +285,7 @@ cudaError_t batch_launch_t(const BatchLaunch<R>& a, int ctas_per_sm, cudaStream_
     if (grid > a.total) grid = a.total > 0 ? a.total : 1;
     *grid_out = (int)grid;
     if (!launch) return cudaSuccess;
-    kern<<<(int)grid, BATCH_NT, smem, s>>>(a);
+    kern<<<(int)grid, batch_nt<R>(), smem, s>>>(a);
     return cudaGetLastError();
 }
 

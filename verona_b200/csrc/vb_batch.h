@@ -8,7 +8,9 @@
 
 namespace VB_NS {
 
-constexpr int BATCH_NT = 256;  // threads per CTA of the batch kernel
+// threads per CTA of the batch kernel: FP64 one cell per thread of a 256-cell tile,
+// FP32 bulk two (vb_tile_pk.cuh)
+template <typename R> constexpr int batch_nt() { return sizeof(R) == 4 ? 128 : 256; }
 constexpr unsigned BATCH_MAX_POLLS = 1u << 24;  // default wait bound, x ~128 ns: a few seconds
 
 struct BatchProb {
