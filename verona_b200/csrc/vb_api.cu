@@ -598,12 +598,19 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
     if (contract && vb_f64c_stage_params_size() != sizeof(StageParams))
         return fail(h, VB_ERR_STATE, "vb_step: FMA-contracted FP64 unit built from another StageParams");
     // the stage's last kernel copies the ghost cells where it has CTAs for them:
-    // the split con2prim kernels, the gated learned form's deferred pass, the 1D / 2D box kernel
+    // the split con2prim kernels, the gated learned form's deferred pass, the 1D / 2D box kernel.
+    // The deferred pass, with few threads per SM, takes them up to a million cells: at 512^3
+    // (4.8 M) it took 250 us with them, 28 us without and k_ghost_limit 205 us
     const bool learned = p.skip_c2p != 0;
-    const bool gated = learned && h->tun.learned_fused != 0 && p.c2p_fp32 && h->defer_idx;
+    const long long ghosts = h->ncell - (long long)h->n[0] * h->n[1] * h->n[2];
+    const bool gated = learned && h->tun.learned_fused != 0 && p.c2p_fp32 && h->defer_idx && ghosts <= (1 << 20);
     const bool last_does_ghosts = learned ? gated : (h->dims < 3 || stage_split_c2p<R>(h->dims, p));
-    p.ghosts = last_does_ghosts && !learned ? ghost_ctas(g, 128) : 0;
-    auto stage = [&](const R* Pin, R* Pout, const double* Us, double* Uo, double dts, double a, double b) -> int {
+    // copy: Pout's ghosts are to become the floored copy of Pin's. Not so in the last of
+    // three stages, whose Pout is the first one's: that stage left them there, and the
+    // floor of a floored value is itself.
+    auto stage = [&](const R* Pin, R* Pout, const double* Us, double* Uo, double dts, double a, double b,
+                     bool copy = true) -> int {
+        p.ghosts = copy && last_does_ghosts && !learned ? ghost_ctas(g, 128) : 0;
         for (int d = 0; d < 3; ++d) p.dtdx[d] = d < h->dims ? dts / h->dx[d] : 0.0;
         p.tmap_in = p.tmap_row = nullptr;
         for (int i = 0; i < 2; ++i) {
@@ -659,7 +666,7 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
                     q.defer_w0 = h->w_guess;
                     VB_CUDA(h, cudaMemsetAsync(h->defer_n, 0, sizeof(unsigned int), s));
                     VB_CUDA(h, launch_c2p_learned<R>(h->mlp_blob, q, bufs, h->tc_err, s));
-                    q.ghosts = ghost_ctas(g, 256);
+                    q.ghosts = copy && last_does_ghosts ? ghost_ctas(g, 256) : 0;
                     VB_CUDA(h, launch_c2p_deferred<R>(q, bufs, s));
                     h->launches += 2;
                 } else {
@@ -674,8 +681,9 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
             }
         }
         if (h->prof) VB_CUDA(h, cudaEventRecord(e1, s));
-        if (!last_does_ghosts) VB_CUDA(h, launch_ghost_limit<R>(g, Pin, Pout, h->opt.floor_, s));
-        h->launches += nk + (last_does_ghosts ? 0 : 1);
+        const bool own = copy && !last_does_ghosts;
+        if (own) VB_CUDA(h, launch_ghost_limit<R>(g, Pin, Pout, h->opt.floor_, s));
+        h->launches += nk + (own ? 1 : 0);
         h->stage_launches += 1;
         return VB_OK;
     };
@@ -684,7 +692,7 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
         // U = 1/3 U + 2/3 (U2 - dt L(P2))
         if ((rc = stage(P[c], P[1 - c], h->U0, h->U1, dt, 0.0, 1.0))) return rc;
         if ((rc = stage(P[1 - c], P[c], h->U1, h->U1, dt, 0.75, 0.25))) return rc;
-        if ((rc = stage(P[c], P[1 - c], h->U1, h->U0, dt, 1.0 / 3.0, 2.0 / 3.0))) return rc;
+        if ((rc = stage(P[c], P[1 - c], h->U1, h->U0, dt, 1.0 / 3.0, 2.0 / 3.0, false))) return rc;
         h->cur = 1 - c;
     } else {
         // midpoint RK2 of the reference: Uhalf = U - dt/2 L(P); U = U - dt L(Phalf)

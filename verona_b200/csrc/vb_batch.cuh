@@ -115,14 +115,18 @@ __device__ __forceinline__ void batch_ghosts(const StageParams& q, const BatchPr
 }
 
 // tile shapes of the kernel variants the autotuner chooses among, and the CTAs per
-// SM that the registers are held to
+// SM that the registers are held to. The tiles wait on barriers, L2 and the serial
+// con2prim, so warps count for more than spills: FP32 (36 tubes + 12 quadrant
+// problems, two steps, a pass) 4, 5, 6, 8 CTAs of 128 threads 5.44, 4.80, 4.33, 4.10
+// ms; FP64 (16 problems of 128^2 to 1024^2, four steps) 2 or 3 of 256 threads 37.2,
+// 34.4 ms.
 template <typename R> struct BatchVariants;
 template <> struct BatchVariants<float> {
-    static constexpr int N = 4, MINB = 4;
+    static constexpr int N = 4, MINB = 8;
     static constexpr int TX2[N] = {32, 32, 64, 16}, TY2[N] = {8, 16, 4, 16}, L1[N] = {256, 512, 128, 256};
 };
 template <> struct BatchVariants<double> {
-    static constexpr int N = 2, MINB = 1;
+    static constexpr int N = 2, MINB = 3;
     static constexpr int TX2[N] = {32, 16}, TY2[N] = {8, 8}, L1[N] = {256, 128};
 };
 

