@@ -245,13 +245,22 @@ template <bool CG, typename T> __device__ __forceinline__ T ld_in(const T* p) {
     return *p;
 }
 
+// the staged ghosts as they are in Pin
+struct KeepHalo {
+    template <typename R>
+    __device__ __forceinline__ void operator()(int, R*) const {}
+};
+
 // One TX x TY x TZ tile of a stage (tile coordinates bx, by, bz); the body of
 // k_stage, shared with the batched kernel. smem_raw: TileGeom::smem_bytes<R>(),
 // or TmaTile2::smem_bytes() for the TMA form (2D; tm: the tensor map of Pin,
-// dims (x, y, variable)), which loads the tile once for both axes.
-template <int DIM, int REC, int RS, typename R, int TX, int TY, int TZ, int NT, bool CG, bool TMA = false>
+// dims (x, y, variable)), which loads the tile once for both axes. halo: called
+// with the tile staged for each axis (not in the TMA form).
+template <int DIM, int REC, int RS, typename R, int TX, int TY, int TZ, int NT, bool CG, bool TMA = false,
+          typename Halo = KeepHalo>
 __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs<R>& b, int bx, int by, int bz,
-                                           unsigned char* smem_raw, const CUtensorMap* tm = nullptr) {
+                                           unsigned char* smem_raw, const CUtensorMap* tm = nullptr,
+                                           const Halo& halo = Halo()) {
     using G = TileGeom<DIM, TX, TY, TZ>;
     using TT = TmaTile2<R, TX, TY>;
     static_assert(!TMA || (DIM == 2 && TZ == 1 && (TX * (int)sizeof(R)) % 16 == 0), "TMA tiles: 2D");
@@ -337,6 +346,7 @@ __device__ __forceinline__ void stage_tile(const StageParams& p, const StageBufs
                 sP[v * EXT + r] = val;
             }
             __syncthreads();
+            halo(d, sP);
         }
         // 2. reconstruct each cell of the tile (plus one halo cell on each side
         //    along d) once; store its two face values, floored. The tile's own

@@ -22,9 +22,9 @@ template <int DIM, int TX, int TY, int NT> struct PkTile {
 };
 
 // one axis: stage the tile with its halo along D, face states, fluxes, differences into sA
-template <int DIM, int D, int REC, int RS, int TX, int TY, int NT>
+template <int DIM, int D, int REC, int RS, int TX, int TY, int NT, typename Halo>
 __device__ __forceinline__ void pk_axis(const StageParams& p, const float* Pin, const int* org, const int* vt,
-                                        double* sA, float* sP, float* sL, float* sR) {
+                                        double* sA, float* sP, float* sL, float* sR, const Halo& halo) {
     using namespace pk;
     constexpr int NV = 2 + DIM, TC = TX * TY;
     constexpr int EX = TX + (D == 0 ? 6 : 0), EY = TY + (D == 1 ? 6 : 0), EXT = EX * EY;
@@ -40,6 +40,7 @@ __device__ __forceinline__ void pk_axis(const StageParams& p, const float* Pin, 
         sP[e] = gi < p.n[0] && gj < p.n[1] ? __ldcg(Pin + v * p.vs + gi + p.sy * gj) : 0.0f;
     }
     __syncthreads();
+    halo(D, sP);
     // the tile's own cells: (lx, ly) with (lx, ly + TY / 2), in 1D lx with lx + TX / 2
     {
         constexpr int DX = DIM == 1 ? TX / 2 : 0, DY = DIM == 1 ? 0 : TY / 2;
@@ -109,9 +110,10 @@ __device__ __forceinline__ void pk_axis(const StageParams& p, const float* Pin, 
     }
 }
 
-template <int DIM, int REC, int RS, int TX, int TY, int NT>
+// halo: called with the tile staged for each axis
+template <int DIM, int REC, int RS, int TX, int TY, int NT, typename Halo>
 __device__ __forceinline__ void stage_tile_pk(const StageParams& p, const StageBufs<float>& b, int bx, int by,
-                                              unsigned char* smem_raw) {
+                                              unsigned char* smem_raw, const Halo& halo) {
     using T = PkTile<DIM, TX, TY, NT>;
     constexpr int NV = 2 + DIM, TC = T::TC;
     double* sA = reinterpret_cast<double*>(smem_raw);
@@ -132,8 +134,8 @@ __device__ __forceinline__ void stage_tile_pk(const StageParams& p, const StageB
 #pragma unroll
             for (int v = 0; v < NV; ++v) sA[v * TC + cell] = __ldcg(b.Us + v * p.vs + c);
     }
-    pk_axis<DIM, 0, REC, RS, TX, TY, NT>(p, b.Pin, org, vt, sA, sP, sL, sR);
-    if constexpr (DIM > 1) pk_axis<DIM, 1, REC, RS, TX, TY, NT>(p, b.Pin, org, vt, sA, sP, sL, sR);
+    pk_axis<DIM, 0, REC, RS, TX, TY, NT>(p, b.Pin, org, vt, sA, sP, sL, sR, halo);
+    if constexpr (DIM > 1) pk_axis<DIM, 1, REC, RS, TX, TY, NT>(p, b.Pin, org, vt, sA, sP, sL, sR, halo);
     unsigned long long n_fail = 0, n_fb = 0, n_it = 0, n_cells = 0;
     for (int cell = tid; cell < TC; cell += NT) {
         long long c;

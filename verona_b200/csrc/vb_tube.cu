@@ -1,7 +1,7 @@
 // Ghosted 1D grids of up to 2048 cells, FP64: every step of a call in one launch
 // of a thread-block cluster. One CTA per 128-cell tile runs the box tile's stage
-// body (stage_tile, vb_stage.cuh) with its loads past L1, edge tiles fill and
-// floor their ghosts as the batch kernel does (batch_ghosts), and the cluster
+// body (stage_tile, vb_stage.cuh) with its loads past L1, the ghosts are filled
+// and floored as in the batch kernel (BatchHalo, batch_ghosts), and the cluster
 // meets once per stage. The kernels of one stage take about as long to launch as
 // to run at this size: N = 1024, MINMOD + HLLC, RK2, 10 steps 377 us in 60 launches,
 // 158 us in one. Longer grids fill the GPU from separate launches and keep
@@ -23,12 +23,11 @@ __device__ __forceinline__ void tube_meet() {
 }
 
 template <int REC, int RS>
-__global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, BatchProb pr, StageParams q) {
+__global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, const __grid_constant__ BatchProb pr, StageParams q) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double t = r.t0;
     int c = r.cur;
     const int stages = r.rk == 3 ? 3 : 2;
-    const bool short_last = pr.ntx > 1 && (pr.n0 - 2 * NG) - (pr.ntx - 1) * TUBE_TX < NG;
     for (int n = 0; n < r.nsteps; ++n, t += r.dt) {
         double *Pc = r.P[c], *Pn = r.P[1 - c];
         for (int st = 0; st < stages; ++st) {
@@ -51,14 +50,9 @@ __global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, BatchProb pr, Stage
             const int tile = (int)blockIdx.x;
             if (tile < pr.ntx) {
                 batch_ghosts<double>(q, pr, b.Pin, b.Pout, tile, 0, TUBE_TX, 1, st == 0, t);
-                __threadfence_block();
-                __syncthreads();
-            }
-            // a last tile of one or two cells leaves the x-hi ghosts that it fills
-            // in the halo of the tile before it
-            if (st == 0 && short_last) tube_meet();
-            if (tile < pr.ntx) {
-                stage_tile<1, REC, RS, double, TUBE_TX, 1, 1, TUBE_TX, true>(q, b, tile, 0, 0, smem_raw);
+                BatchHalo<double> halo;
+                halo.init(pr, b.Pin, tile, 0, TUBE_TX, 1, st == 0, t);
+                stage_tile<1, REC, RS, double, TUBE_TX, 1, 1, TUBE_TX, true>(q, b, tile, 0, 0, smem_raw, nullptr, halo);
             }
             tube_meet();
         }
