@@ -17,13 +17,13 @@
 // Compiled with -fmad=false: bit-identical to the oracle restatement.
 #include <algorithm>
 
+#include "vb_cluster.cuh"
 #include "vb_con2prim.cuh"
 #include "vb_internal.h"
 
 namespace vb {
 
 constexpr int R1_MAXT = 480;     // threads per CTA: cells of a tile + 2 (46 KB of shared memory)
-constexpr int R1_CLUSTER = 16;   // CTAs, where the GPU grants such a cluster; else 8 (portable)
 
 __device__ __forceinline__ void ref1d_cons(double g, double p1, double p2, double p3, double* U) {
     double gamma = sqrt(sq(p3) + 1.0);
@@ -113,12 +113,6 @@ __device__ __forceinline__ void ref1d_hll(double g, const double* pl, const doub
 #pragma unroll
         for (int v = 0; v < 3; ++v) F[v] = f[v];
     }
-}
-
-__device__ __forceinline__ void cluster_meet() {
-    __threadfence();  // this thread's stores of P before the others' loads
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // One RK stage of cells [a, b): face states and fluxes of P (faces a-1 .. b-1),
@@ -248,36 +242,14 @@ template <int REC>
 static cudaError_t launch_ref1d_rec(const Ref1DState& st, double g, int n_iter, double tol, double dt, double dx,
                                     int nsteps, cudaStream_t s) {
     auto kern = k_ref1d_steps<REC>;
-    static int widest[64] = {0};  // largest cluster per device; racing writers store the same value
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& wide = widest[dev & 63];
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    if (!wide) {
-        int fit = 0;
-        at.val.clusterDim.x = R1_CLUSTER;
-        cfg.gridDim = dim3(R1_CLUSTER);
-        cfg.blockDim = dim3(R1_MAXT);
-        const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0;
-        if (!ok) cudaGetLastError();  // a refused cluster size is no error of this call
-        wide = ok ? R1_CLUSTER : 8;
-    }
+    static int widest[64] = {0};
+    const int wide = widest_cluster(kern, R1_MAXT, 0, widest);
     // at least 32 cells per CTA
     int c = 1;
     while (c < wide && 64 * c <= st.N) c *= 2;
     const int m = (st.N + c - 1) / c;
     const int t = std::min(R1_MAXT, (m + 2 + 31) / 32 * 32);
-    at.val.clusterDim.x = c;
-    cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(t);
-    return cudaLaunchKernelEx(&cfg, kern, st, g, n_iter, tol, dt, dx, nsteps);
+    return launch_cluster(kern, c, t, 0, s, st, g, n_iter, tol, dt, dx, nsteps);
 }
 
 cudaError_t launch_ref1d_steps(const Ref1DState& st, double g, int rec, int n_iter, double tol, double dt,

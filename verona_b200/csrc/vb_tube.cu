@@ -10,17 +10,12 @@
 #include <cstring>
 
 #include "vb_batch.cuh"
+#include "vb_cluster.cuh"
 #include "vb_tube.h"
 
 namespace vb {
 
-constexpr int TUBE_TX = 128, TUBE_CLUSTER = 16;
-
-__device__ __forceinline__ void tube_meet() {
-    __threadfence();  // this thread's stores before the other CTAs' loads
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+constexpr int TUBE_TX = 128;
 
 template <int REC, int RS>
 __global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, const __grid_constant__ BatchProb pr, StageParams q) {
@@ -54,46 +49,23 @@ __global__ void __launch_bounds__(TUBE_TX) k_tube(TubeRun r, const __grid_consta
                 halo.init(pr, b.Pin, tile, 0, TUBE_TX, 1, st == 0, t);
                 stage_tile<1, REC, RS, double, TUBE_TX, 1, 1, TUBE_TX, true>(q, b, tile, 0, 0, smem_raw, nullptr, halo);
             }
-            tube_meet();
+            cluster_meet();
         }
         if (r.rk == 3) c ^= 1;  // an odd number of buffer swaps
     }
 }
 
-bool tube_fits(int cells) { return cells <= TUBE_TX * TUBE_CLUSTER; }
+bool tube_fits(int cells) { return cells <= TUBE_TX * CLUSTER_MAX; }
 
 template <int REC, int RS>
 static cudaError_t launch_tube_t(const TubeRun& r, const BatchProb& pr, const StageParams& q, cudaStream_t s) {
     auto kern = k_tube<REC, RS>;
     constexpr size_t smem = TileGeom<1, TUBE_TX, 1, 1>::smem_bytes<double>();
-    static int widest[64] = {0};  // largest cluster per device; racing writers store the same value
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& wide = widest[dev & 63];
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cfg.blockDim = dim3(TUBE_TX);
-    cfg.dynamicSmemBytes = smem;
-    if (!wide) {
-        int fit = 0;
-        at.val.clusterDim.x = TUBE_CLUSTER;
-        cfg.gridDim = dim3(TUBE_CLUSTER);
-        const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0;
-        if (!ok) cudaGetLastError();
-        wide = ok ? TUBE_CLUSTER : 8;
-    }
+    static int widest[64] = {0};
     int c = 1;
     while (c < pr.ntx) c *= 2;
-    if (c > wide) return cudaErrorNotSupported;  // the caller takes the separate kernels
-    at.val.clusterDim.x = c;
-    cfg.gridDim = dim3(c);
-    return cudaLaunchKernelEx(&cfg, kern, r, pr, q);
+    if (c > widest_cluster(kern, TUBE_TX, smem, widest)) return cudaErrorNotSupported;  // the caller takes the separate kernels
+    return launch_cluster(kern, c, TUBE_TX, smem, s, r, pr, q);
 }
 
 cudaError_t launch_tube(int rec, int rs, const TubeRun& r, const int* bc_kind, const double (*bc_par)[16],
