@@ -15,11 +15,15 @@
 // Rows arrive in a ring of eight per warp, [4 variables][40 columns] each: by
 // TMA (one box per row, two rows ahead; the box starts at the 16-byte boundary
 // at or before the strip), or by 4-byte asynchronous copies (tma_tiles = 0).
-// The kernel writes U = rk_a U0 + rk_b (Us - div) in FP64 from the FP32
-// divergence; con2prim follows in k_c2p_2d. Scheme: src/2dim/algos.jl:11-189.
+// The kernel writes U = rk_a U0 + rk_b (Us - div) with the flux differences of the
+// FP32 fluxes and their sum in FP64, as the box kernel does: a face's flux leaves
+// one cell and enters the next with the same FP64 factor, so sums of U over the grid
+// keep to FP64 rounding. con2prim follows in k_c2p_2d. Scheme: src/2dim/algos.jl:11-189.
 //
-// 2047 x 1021, WENOZ + HLLC: 91 us a stage against 237 us of the box kernel, both
-// without con2prim (con2prim apart: 47 us).
+// 2047 x 1021, WENOZ + HLLC: 102 us a stage against 239 us of the box kernel, both
+// without con2prim (con2prim apart: 51 us); 4096 x 4096: 0.67 ms. With the divergence
+// summed in FP32 it took 92 us: the FP64 sums are 28 conversions, an eighth of
+// the FP32 rate each, for 8 values.
 #pragma once
 #include "vb_ns.h"
 #include <cuda.h>  // CUtensorMap
@@ -160,10 +164,12 @@ __global__ void __launch_bounds__(YpGeom::NT, MINB)
                 }
             }
         }
-        f2 acc[NV];
+        // fluxes of the faces left of the cell (x) and, below, above it (y); their
+        // differences wait for the end of the step, where no state is live
+        f2 Fx[NV], Fy[NV];
         {  // x
             const float *ra = row(j) + o, *rb = row(j + 1) + o;
-            f2 qr[NV], L[NV], F[NV];
+            f2 qr[NV], L[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 const int k = v * BXW;
@@ -176,41 +182,35 @@ __global__ void __launch_bounds__(YpGeom::NT, MINB)
                 }
                 L[v] = P2(__shfl_up_sync(0xffffffffu, ql.x, 1), __shfl_up_sync(0xffffffffu, ql.y, 1));
             }
-            face_flux<0, RS, 2>(g, gm1, L, qr, F);
-            const f2 cx = S2((float)p.dtdx[0]);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const f2 Fr = P2(__shfl_down_sync(0xffffffffu, F[v].x, 1), __shfl_down_sync(0xffffffffu, F[v].y, 1));
-                acc[v] = mul(cx, sub(Fr, F[v]));
-            }
+            face_flux<0, RS, 2>(g, gm1, L, qr, Fx);
         }
         {  // y: rows j+1, j+2 from the rows j-1 .. j+4; faces j+1/2, j+3/2
-            f2 qr[NV], ql[NV], L[NV], F[NV];
+            f2 qr[NV], ql[NV], L[NV];
             yrecon(j + 1, qr, ql);
 #pragma unroll
             for (int v = 0; v < NV; ++v) L[v] = P2(qly[v], ql[v].x);
-            face_flux<1, RS, 2>(g, gm1, L, qr, F);
-            const f2 cy = S2((float)p.dtdx[1]);
+            face_flux<1, RS, 2>(g, gm1, L, qr, Fy);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                acc[v] = fma(cy, sub(F[v], P2(Fym[v], F[v].x)), acc[v]);
-                Fym[v] = F[v].y;
-                qly[v] = ql[v].y;
-            }
+            for (int v = 0; v < NV; ++v) qly[v] = ql[v].y;
         }
         cp_async_wait_all();
-        if (mine) {
-            double* out = b.Uo + (x + sy * j);
+        const double cx = p.dtdx[0], cy = p.dtdx[1];
+        double* out = b.Uo + (x + sy * j);
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                if (q == 1 && !two) break;
+        for (int v = 0; v < NV; ++v) {
+            const float rx = __shfl_down_sync(0xffffffffu, Fx[v].x, 1), ry = __shfl_down_sync(0xffffffffu, Fx[v].y, 1);
+            if (mine) {
 #pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    double u = ubuf[(q * NV + v) * 32] - (double)(q ? acc[v].y : acc[v].x);
+                for (int q = 0; q < 2; ++q) {
+                    if (q == 1 && !two) break;
+                    double u = ubuf[(q * NV + v) * 32];
+                    u = u - cx * ((double)(q ? ry : rx) - (double)(q ? Fx[v].y : Fx[v].x));
+                    u = u - cy * ((double)(q ? Fy[v].y : Fy[v].x) - (double)(q ? Fy[v].x : Fym[v]));
                     if (p.rk_a != 0.0) u = p.rk_a * ubuf[((2 + q) * NV + v) * 32] + p.rk_b * u;
                     out[v * vs + q * sy] = u;
                 }
             }
+            Fym[v] = Fy[v].y;
         }
         if (j + 2 < yend) {
             if constexpr (TMA) {
