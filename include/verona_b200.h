@@ -225,7 +225,9 @@ int vb_reset_counters(vb_handle h, void* stream);
  * 1 = the z-pair (3D) or y-marching (2D) stencil kernel, two cells per thread on
  * packed FP32 pairs (in 2D con2prim then runs in a kernel of its own, whatever
  * split_con2prim); 0 = one cell per thread; -1 = library default (1). The two
- * agree to FP32 rounding, not bitwise.
+ * agree to FP32 rounding, not bitwise. 3D grids of whole 32 x 8 column tiles sum the
+ * flux differences in FP32; 2D grids and 3D grids with a ragged tile in FP64, the
+ * latter by the box kernel where fp32_pairs = 0 or split_con2prim = 0.
  * tma_tiles: 1 = the stencil kernels stage the state in shared memory as TMA
  * tiles (cp.async.bulk.tensor): in 3D (FP32 bulk, z-pair kernel) every plane
  * with its x/y halo, a ring of 6 planes per CTA; in 2D FP32 bulk every row of a

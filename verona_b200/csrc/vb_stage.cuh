@@ -568,10 +568,11 @@ cudaError_t dispatch_stage_dim(int rec, int rs, const StageParams& p, const Stag
     return cudaErrorInvalidValue;
 }
 
+template <typename R> bool zm_used(const StageParams& p);
 template <typename R>
 cudaError_t dispatch_stage_zm(int rec, int rs, const StageParams& p, const StageBufs<R>& b, cudaStream_t s);
 
-// 3D grids use the z-marching kernels (unless force_box) and 2D FP32-bulk grids
+// 3D grids use the z-marching kernels (where zm_used) and 2D FP32-bulk grids
 // the y-marching one (unless pairs = 0); 1D and 2D FP64 the box-tile k_stage.
 // *kernels receives the number of kernels launched (2 for a split z-march
 // stage, whose con2prim runs in k_c2p; else 1).
@@ -601,7 +602,7 @@ cudaError_t launch_stage(int dims, int rec, int rs, const StageParams& p, const 
         return launch_c2p<R>(p, b, s);
     }
     if (dims == 3) {
-        if (!p.force_box) {
+        if (zm_used<R>(p)) {
             *kernels = p.split && !p.skip_c2p ? 2 : 1;
             return dispatch_stage_zm<R>(rec, rs, p, b, s);
         }

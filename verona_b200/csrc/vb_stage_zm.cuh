@@ -340,6 +340,21 @@ template <typename R> struct ZmCfg;
 template <> struct ZmCfg<float> { static constexpr int TX = 32, TY = 8, MINB = 3, MINB_SPLIT = 4; };
 template <> struct ZmCfg<double> { static constexpr int TX = 32, TY = 8, MINB = 2, MINB_SPLIT = 2; };
 
+// every column tile whole
+template <typename R> inline bool zm_whole(const StageParams& p) {
+    using C = ZmCfg<R>;
+    return (p.n[0] - 2 * NG) % C::TX == 0 && (p.n[1] - 2 * NG) % C::TY == 0;
+}
+// The z-marching kernels do this 3D stage, else the box kernel. In FP32 bulk a
+// ragged grid's flux differences are summed in FP64, as the box kernel sums them,
+// which only the z-pair kernel that writes U offers (300 x 125 x 125, WENOZ + HLLC,
+// a stencil launch: 0.44 ms, 0.35 with FP32 sums and the divergence handed on,
+// 2.06 ms of the box kernel).
+template <typename R> bool zm_used(const StageParams& p) {
+    if (p.force_box) return false;
+    return std::is_same<R, double>::value || zm_whole<R>(p) || (p.pairs && (p.split || p.skip_c2p));
+}
+
 // Planes per z range of a z-marching kernel. A range costs its planes plus a
 // prologue (the window's loads, two reconstructions and one flux: 0.6 planes),
 // and CTAs run on `slots` places: x = CTAs / slots rounds of them take between
@@ -570,7 +585,7 @@ cudaError_t launch_stage_zm(const StageParams& p, const StageBufs<R>& b, cudaStr
 }
 
 template <typename R> int stage_div_in_pout(int dims, int rec, int rs, const StageParams& p) {
-    if (!std::is_same<R, float>::value || dims != 3 || p.force_box) return 0;
+    if (!std::is_same<R, float>::value || dims != 3 || p.force_box || !zm_whole<R>(p)) return 0;
     return p.pairs && zp_available(rec, rs) && p.skip_c2p && p.want_div ? 1 : 0;
 }
 
@@ -583,7 +598,7 @@ template <typename R> int stage_split_c2p(int dims, const StageParams& p) {
         const bool yp = std::is_same<R, float>::value && p.pairs;
         return (p.split || yp) && !p.skip_c2p ? 1 : 0;
     }
-    return dims == 3 && !p.force_box && p.split && !p.skip_c2p ? 1 : 0;
+    return dims == 3 && zm_used<R>(p) && p.split && !p.skip_c2p ? 1 : 0;
 }
 
 template <typename R>

@@ -441,11 +441,17 @@ enum { ZP_FUSED = 0, ZP_U = 1, ZP_DIV = 2 };
 // the tensor map of Pin, dims (x, y, z, variable)); otherwise the column's
 // z-window is loaded by the thread and the x/y halo of the planes (k, k+1)
 // by 4-byte asynchronous copies into an interleaved pair buffer.
-// FULL: every tile is whole and every range has Z_RANGE_MAX planes, known at
-// compile time; the general form, whose edge tiles test each column and whose
-// ranges have lz planes, takes 2 % longer on a large grid of whole tiles (512^3
-// WENOZ + HLLC, divergence out: 8.17 against 8.01 ms), so such grids use FULL.
-template <int REC, int RS, int TX, int TY, int MINB, int TAIL, bool TMA, bool FULL>
+// GRID: ZG_WHOLE, every tile whole, ranges of lz planes; ZG_FULL, moreover every
+// range Z_RANGE_MAX planes, known at compile time (512^3 WENOZ + HLLC,
+// divergence out: 8.02 ms, 8.17 with range and columns tested at run time);
+// ZG_RAGGED, tiles of the last column or row past the interior. ZG_RAGGED writes U
+// (TAIL = ZP_U) with the flux differences of the FP32 fluxes and their sum in FP64, as
+// the box kernel, the other form that such grids have, does; ZG_WHOLE and ZG_FULL
+// sum the divergence in FP32 as k_stage_zm does. So that no FP64 sum stays in
+// registers through the phases, the x fluxes of ZG_RAGGED keep a buffer of their
+// own, and every difference is formed at the end of the pair.
+enum { ZG_RAGGED = 0, ZG_WHOLE = 1, ZG_FULL = 2 };
+template <int REC, int RS, int TX, int TY, int MINB, int TAIL, bool TMA, int GRID>
 __global__ void __launch_bounds__(TX * TY, MINB)
     k_stage_zp(StageParams p, StageBufs<float> b, int lz_, const __grid_constant__ CUtensorMap tm) {
     using namespace pk;
@@ -456,12 +462,15 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     // plane access: element (v, y, x) of a plane at v * VSTR + (y + 3) * ROW + x + 3
     constexpr int ROW = TMA ? TG::BXW : G::EX, VSTR = TMA ? TG::VSTR : G::PLN, SLOTF = TG::SLOTF;
     static_assert(!TMA || TX % 4 == 0, "TMA boxes start at x = TX * blockIdx.x");
+    static_assert(GRID != ZG_RAGGED || TAIL == ZP_U, "ragged tiles: U out");
+    constexpr bool WIDE = GRID == ZG_RAGGED;  // FP64 sums
     extern __shared__ __align__(16) unsigned char smem_raw[];  // TMA form: 128-byte base found below
     f2* sPl = nullptr;         // cp.async form: [NV][EY][EX] planes (k, k+1) with x/y halo
     float* sZ = nullptr;       // cp.async form: [ZR][NV][NT] this thread's z-window
     float* sRing = nullptr;    // TMA form: [ZR][SLOTF] plane boxes
     uint64_t* sBar = nullptr;  // TMA form: one mbarrier per ring slot
-    f2 *sQL, *sF, *sQX;        // [NV][FN] left states, [NV][FN] fluxes, [NV][QXN] last right states
+    f2 *sQL, *sF, *sQX;        // [NV][FN] left states, [NV][FN] fluxes (WIDE: y), [NV][QXN] last right states
+    f2* sFX;                   // x fluxes; WIDE: [NV][FN] of their own
     f2* sYH;                   // [NV][2 TX]: ql of the cells of row -1, qr of the cells of row TY
     if constexpr (TMA) {
         unsigned char* base = smem_raw + ((128u - (tc::smem_u32(smem_raw) & 127u)) & 127u);
@@ -470,14 +479,16 @@ __global__ void __launch_bounds__(TX * TY, MINB)
         sF = sQL + NV * FN;
         sQX = sF + NV * FN;
         sYH = sQX + NV * QXN;
-        sBar = reinterpret_cast<uint64_t*>(sYH + NV * G::YHN);
+        sFX = WIDE ? sYH + NV * G::YHN : sF;
+        sBar = reinterpret_cast<uint64_t*>(WIDE ? sFX + NV * FN : sYH + NV * G::YHN);
     } else {
         sPl = reinterpret_cast<f2*>(smem_raw);
         sQL = sPl + NV * G::PLN;
         sF = sQL + NV * FN;
         sQX = sF + NV * FN;
         sYH = sQX + NV * QXN;
-        sZ = reinterpret_cast<float*>(sYH + NV * G::YHN);
+        sFX = WIDE ? sYH + NV * G::YHN : sF;
+        sZ = reinterpret_cast<float*>(WIDE ? sFX + NV * FN : sYH + NV * G::YHN);
     }
 
     const int tid = threadIdx.x;
@@ -487,8 +498,9 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     // padded column; only interior columns (mine) touch U and the output
     const int ilast = p.n[0] - 1, jlast = p.n[1] - 1;
     const int i = TMA ? i0 + tx : min(i0 + tx, ilast), j = TMA ? j0 + ty : min(j0 + ty, jlast);
-    const bool mine = FULL || (i0 + tx < p.n[0] - NG && j0 + ty < p.n[1] - NG);
-    const int lz = FULL ? Z_RANGE_MAX : lz_;
+    // (ZG_WHOLE's are all interior; without the test its ZP_U form took 0.5 % longer)
+    const bool mine = GRID == ZG_FULL || TAIL == ZP_DIV || (i0 + tx < p.n[0] - NG && j0 + ty < p.n[1] - NG);
+    const int lz = GRID == ZG_FULL ? Z_RANGE_MAX : lz_;
     const int z0 = NG + blockIdx.z * lz;
     const int zend = min(z0 + lz, p.n[2] - NG);
     const long long sy = p.sy, sz = p.sz, vs = p.vs;
@@ -690,7 +702,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
             for (int v = 0; v < NV; ++v) PL[v] = sQL[v * FN + ty * FXR + tx];
             face_flux<0, RS>(g, gm1, PL, qrx, F);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) sF[v * FN + ty * FXR + tx] = F[v];
+            for (int v = 0; v < NV; ++v) sFX[v * FN + ty * FXR + tx] = F[v];
         }
         // the last warp computes the TY faces at the tiles' x edge; meanwhile the
         // other warps reconstruct the y halo (cells -1 and TY of every column,
@@ -708,7 +720,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
                 }
                 face_flux<0, RS>(g, gm1, PL, PR, F);
 #pragma unroll
-                for (int v = 0; v < NV; ++v) sF[v * FN + e * FXR + TX] = F[v];
+                for (int v = 0; v < NV; ++v) sFX[v * FN + e * FXR + TX] = F[v];
             }
         } else {
             for (int e = tid; e < 2 * TX * NV; e += NT - 32) {
@@ -725,9 +737,11 @@ __global__ void __launch_bounds__(TX * TY, MINB)
             }
         }
         __syncthreads();
+        if constexpr (!WIDE) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v)
-            acc[v] = fma(cx, sub(sF[v * FN + ty * FXR + tx + 1], sF[v * FN + ty * FXR + tx]), acc[v]);
+            for (int v = 0; v < NV; ++v)
+                acc[v] = fma(cx, sub(sF[v * FN + ty * FXR + tx + 1], sF[v * FN + ty * FXR + tx]), acc[v]);
+        }
 
         // y: reconstruct own cells; halo cells -1 and TY of each column
         f2 qry[NV];
@@ -771,9 +785,11 @@ __global__ void __launch_bounds__(TX * TY, MINB)
             for (int v = 0; v < NV; ++v) sF[v * FN + TY * TX + e] = F[v];
         }
         __syncthreads();
+        if constexpr (!WIDE) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v)
-            acc[v] = fma(cy, sub(sF[v * FN + (ty + 1) * TX + tx], sF[v * FN + ty * TX + tx]), acc[v]);
+            for (int v = 0; v < NV; ++v)
+                acc[v] = fma(cy, sub(sF[v * FN + (ty + 1) * TX + tx], sF[v * FN + ty * TX + tx]), acc[v]);
+        }
 
         // z: planes k+5, k+6 are fetched now and enter the window after the
         // reconstruction of cells (k+1, k+2) from planes k-1 .. k+4; faces
@@ -797,15 +813,17 @@ __global__ void __launch_bounds__(TX * TY, MINB)
             Pk[v] = zs(k, v);
             Pk[NV + v] = zs(k + 1, v);
         }
+        f2 Fzl[NV], Fz[NV];  // fluxes below and above the two cells
         {
-            f2 qr1[NV], ql1[NV], L[NV], Fz[NV];
+            f2 qr1[NV], ql1[NV], L[NV];
             zrecon(k + 1, qr1, ql1);
 #pragma unroll
             for (int v = 0; v < NV; ++v) L[v] = P2(qlz[v], ql1[v].x);
             face_flux<2, RS>(g, gm1, L, qr1, Fz);
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                acc[v] = fma(cz, sub(Fz[v], P2(Fzm[v], Fz[v].x)), acc[v]);
+                Fzl[v] = P2(Fzm[v], Fz[v].x);
+                if (!WIDE) acc[v] = fma(cz, sub(Fz[v], Fzl[v]), acc[v]);
                 Fzm[v] = Fz[v].y;
                 qlz[v] = ql1[v].y;
             }
@@ -820,28 +838,23 @@ __global__ void __launch_bounds__(TX * TY, MINB)
         // ZP_DIV: the FP32 divergence into Pout; ZP_U: the RK combination in FP64
         // (U - div) into Uo; ZP_FUSED: that, then con2prim (guess: this stage's P)
         // and the floors
-        if (TAIL == ZP_DIV && FULL) {
+        if (TAIL == ZP_DIV) {
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 b.Pout[v * vs + c] = acc[v].x;
                 if (two) b.Pout[v * vs + c + sz] = acc[v].y;
             }
-        } else if (TAIL == ZP_DIV) {
-            // the column again from the thread index: kept across the loop it
-            // cost registers (8.26 against 8.17 ms per 512^3 launch)
-            int t;
-            asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
-            const int io = i0 + t % TX, jo = j0 + t / TX;
-            if (io < p.n[0] - NG && jo < p.n[1] - NG) {
-                float* o = b.Pout + (io + sy * jo + sz * k);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    o[0] = acc[v].x;
-                    if (two) o[sz] = acc[v].y;
-                    o += vs;
-                }
-            }
         }
+        // WIDE: Us - dt/dx (F_hi - F_lo) axis by axis in FP64
+        auto wide_u = [&](double u, int v, int q) -> double {
+            auto sub_axis = [&](double cdt, f2 hi, f2 lo) {
+                u = u - cdt * ((double)(q ? hi.y : hi.x) - (double)(q ? lo.y : lo.x));
+            };
+            sub_axis(p.dtdx[0], sFX[v * FN + ty * FXR + tx + 1], sFX[v * FN + ty * FXR + tx]);
+            sub_axis(p.dtdx[1], sF[v * FN + (ty + 1) * TX + tx], sF[v * FN + ty * TX + tx]);
+            sub_axis(p.dtdx[2], Fz[v], Fzl[v]);
+            return u;
+        };
 #pragma unroll
         for (int q = 0; q < (TAIL == ZP_DIV ? 0 : 2); ++q) {
             if (!mine || (q == 1 && !two)) break;
@@ -849,7 +862,11 @@ __global__ void __launch_bounds__(TX * TY, MINB)
             double U[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                double u = b.Us[v * vs + cc] - (double)(q ? acc[v].y : acc[v].x);
+                double u = b.Us[v * vs + cc];
+                if constexpr (WIDE)
+                    u = wide_u(u, v, q);
+                else
+                    u = u - (double)(q ? acc[v].y : acc[v].x);
                 if (p.rk_a != 0.0) u = p.rk_a * b.U0[v * vs + cc] + p.rk_b * u;
                 U[v] = u;
                 b.Uo[v * vs + cc] = u;
@@ -904,12 +921,15 @@ struct ZpCfg {
     static constexpr int TX = 32, TY = 8, MINB = 2, MINB_SPLIT = 2;
 };
 
-template <int REC, int RS, int TAIL, bool TMA, bool FULL>
+template <int REC, int RS, int TAIL, bool TMA, int GRID>
 cudaError_t launch_stage_zp_g(const StageParams& p, const StageBufs<float>& b, dim3 grid, int lz, cudaStream_t s) {
     using C = ZpCfg;
     constexpr int MINB = TAIL == ZP_FUSED ? C::MINB : C::MINB_SPLIT;
-    auto kern = k_stage_zp<REC, RS, C::TX, C::TY, MINB, TAIL, TMA, FULL>;
-    constexpr size_t smem = TMA ? ZpTmaGeom<C::TX, C::TY>::smem_bytes() : ZpGeom<C::TX, C::TY>::smem_bytes();
+    auto kern = k_stage_zp<REC, RS, C::TX, C::TY, MINB, TAIL, TMA, GRID>;
+    using G = ZpGeom<C::TX, C::TY>;
+    constexpr size_t smem = (TMA ? ZpTmaGeom<C::TX, C::TY>::smem_bytes() : G::smem_bytes()) +
+                            (GRID == ZG_RAGGED ? sizeof(float2) * G::NV * G::FN : 0);
+    static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM");
     static unsigned long long attr_set = 0;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -936,20 +956,23 @@ cudaError_t launch_stage_zp_t(const StageParams& p, const StageBufs<float>& b, c
     using C = ZpCfg;
     int lz;
     const dim3 grid = z_march_grid(p, C::TX, C::TY, TAIL == ZP_FUSED ? C::MINB : C::MINB_SPLIT, 2, &lz);
-    if constexpr (TMA && TAIL != ZP_FUSED) {
-        const bool whole = (p.n[0] - 2 * NG) % C::TX == 0 && (p.n[1] - 2 * NG) % C::TY == 0;
-        if (whole && lz == Z_RANGE_MAX) return launch_stage_zp_g<REC, RS, TAIL, TMA, true>(p, b, grid, lz, s);
+    if (!zm_whole<float>(p)) {
+        if constexpr (TAIL == ZP_U) return launch_stage_zp_g<REC, RS, TAIL, TMA, ZG_RAGGED>(p, b, grid, lz, s);
+        return cudaErrorInvalidValue;  // launch_stage takes such grids elsewhere
     }
-    return launch_stage_zp_g<REC, RS, TAIL, TMA, false>(p, b, grid, lz, s);
+    if constexpr (TMA && TAIL != ZP_FUSED) {
+        if (lz == Z_RANGE_MAX) return launch_stage_zp_g<REC, RS, TAIL, TMA, ZG_FULL>(p, b, grid, lz, s);
+    }
+    return launch_stage_zp_g<REC, RS, TAIL, TMA, ZG_WHOLE>(p, b, grid, lz, s);
 }
 
 // Every reconstruction with HLL or HLLC in the FP32-bulk form (zp_available).
 // The divergence hand-off (ZP_DIV) is taken when the caller's con2prim kernel
-// forms U itself (p.want_div, the fused learned con2prim).
+// forms U itself (p.want_div, the fused learned con2prim) and the tiles are whole.
 template <int REC, int RS, bool TMA>
 cudaError_t dispatch_stage_zp_tail(const StageParams& p, const StageBufs<float>& b, cudaStream_t s) {
     if (!(p.split || p.skip_c2p)) return launch_stage_zp_t<REC, RS, ZP_FUSED, TMA>(p, b, s);
-    if (p.skip_c2p && p.want_div) return launch_stage_zp_t<REC, RS, ZP_DIV, TMA>(p, b, s);
+    if (p.skip_c2p && p.want_div && zm_whole<float>(p)) return launch_stage_zp_t<REC, RS, ZP_DIV, TMA>(p, b, s);
     return launch_stage_zp_t<REC, RS, ZP_U, TMA>(p, b, s);
 }
 // the TMA form where the caller encoded a tensor map of Pin (p.tmap_in)
