@@ -453,7 +453,8 @@ int vb_batch_reset_counters(vb_batch_handle b, void* stream);
 /* tile variants of a precision (0 for an invalid precision) and their shapes */
 int vb_batch_num_variants(int precision);
 int vb_batch_variant_shape(int precision, int variant, int* tile_x2, int* tile_y2, int* pencil1);
-/* ctas_per_sm 0: as many as fit; the grid of the last launch is returned by get */
+/* ctas_per_sm: CTAs of 256 threads (the FP32-bulk kernel runs two of 128 for each),
+ * 0: as many as fit; the grid of the last launch is returned by get */
 int vb_batch_set_tuning(vb_batch_handle b, int variant, int ctas_per_sm);
 int vb_batch_get_tuning(vb_batch_handle b, int* variant, int* ctas_per_sm, int* grid);
 int vb_batch_info(vb_batch_handle b, int64_t* interior_cells, int64_t* tiles_per_stage, int64_t* device_bytes);

@@ -3,8 +3,9 @@ shape) and CTAs per SM of one persistent launch.
 
 A grid search over the candidates, timed with CUDA events on the batch's own
 problems; the batch state is checkpointed before and restored after, so
-tuning leaves the solution unchanged. Results are cached per (GPU, batch
-signature) in a JSON file: $VB_TUNE_CACHE, else ~/.cache/verona_b200/batch_tuning.json.
+tuning leaves the solution unchanged. Results are cached per (GPU, kernel
+generation, batch signature) in a JSON file: $VB_TUNE_CACHE, else
+~/.cache/verona_b200/batch_tuning.json.
 """
 from __future__ import annotations
 
@@ -12,6 +13,11 @@ import json
 import os
 
 from .batch import Batch, variants
+
+
+# Raised whenever the batch kernel's tiles, threads or registers change, so that a
+# choice made for an older kernel is made again. 2: FP32 tiles on packed pairs.
+KERNEL_GENERATION = 2
 
 
 def cache_path() -> str:
@@ -34,14 +40,14 @@ def _gpu_key():
     return f"{p.name}/sm{p.major}{p.minor}/{p.multi_processor_count}"
 
 
-def tune_batch(b: Batch, steps: int = 2, ctas_candidates=(0, 1, 2), use_cache: bool = True, path: str | None = None,
+def tune_batch(b: Batch, steps: int = 2, ctas_candidates=(0, 1, 2, 3), use_cache: bool = True, path: str | None = None,
                log=None) -> dict:
     """Pick and apply the fastest (variant, CTAs per SM); returns the choice
     with the timings of every candidate (ms per step)."""
     import torch
 
     path = path or cache_path()
-    key = f"{_gpu_key()}/{b.signature()}"
+    key = f"{_gpu_key()}/k{KERNEL_GENERATION}/{b.signature()}"
     if use_cache:
         hit = _load(path).get(key)
         if hit:

@@ -325,7 +325,9 @@ cudaError_t batch_launch_t(const BatchLaunch<R>& a, int ctas_per_sm, cudaStream_
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, kern, batch_nt<R>(), smem);
     if (e != cudaSuccess) return e;
     if (maxb < 1) return cudaErrorInvalidConfiguration;
-    const int per = ctas_per_sm > 0 ? std::min(ctas_per_sm, maxb) : maxb;
+    // the caller's CTAs are of 256 threads; the FP32 kernel takes two of 128 for each
+    constexpr int unit = BATCH_CTA / batch_nt<R>();
+    const int per = ctas_per_sm > 0 ? std::min(ctas_per_sm * unit, maxb) : maxb;
     long long grid = (long long)per * nsm;
     if (grid > a.total) grid = a.total > 0 ? a.total : 1;
     *grid_out = (int)grid;

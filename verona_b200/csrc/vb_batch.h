@@ -11,6 +11,7 @@ namespace VB_NS {
 // threads per CTA of the batch kernel: FP64 one cell per thread of a 256-cell tile,
 // FP32 bulk two (vb_tile_pk.cuh)
 template <typename R> constexpr int batch_nt() { return sizeof(R) == 4 ? 128 : 256; }
+constexpr int BATCH_CTA = 256;  // threads of a CTA as vb_batch_set_tuning counts them
 constexpr unsigned BATCH_MAX_POLLS = 1u << 24;  // default wait bound, x ~128 ns: a few seconds
 
 struct BatchProb {
