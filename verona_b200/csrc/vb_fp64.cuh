@@ -39,7 +39,7 @@
 // tests/fp64_range_check.cu draws operands over all of that range and, by
 // construction, quotients and roots next to a middle: of 1e10 trials of each kind
 // none differs from the IEEE operation at 2^-51 ulp or more from a middle, 184 of
-// about 1e9 nearer do, by one ulp.
+// some 3e9 nearer do, by one ulp.
 #pragma once
 #include "vb_ns.h"
 #include <cuda_runtime.h>
