@@ -6,7 +6,8 @@ Translation units and their floating-point contract:
   vb_stage_f64c.cu                          -fmad=true   (the FP64 stage kernels with FMA
                                             contraction, namespace vb_f64c; tuning
                                             fp64_contract)
-  vb_stage_f32.cu, vb_stage_yp_f32.cu       -fmad=true, approximate FP32 divide and
+  vb_stage_f32.cu, vb_stage_yp_f32.cu, vb_stage_zp_f32.cu
+                                            -fmad=true, approximate FP32 divide and
                                             square root, FTZ (FP32-bulk path; the
                                             FP64 con2prim in it stays IEEE)
   vb_mlp.cu                                 -fmad=true   (BF16 tensor-core MLP)
@@ -39,6 +40,7 @@ UNITS = {
     "vb_tube.cu": ["-fmad=false"],
     "vb_api.cu": ["-fmad=false"],
     "vb_stage_f32.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
+    "vb_stage_zp_f32.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
     "vb_stage_yp_f32.cu": ["-fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
 }
 

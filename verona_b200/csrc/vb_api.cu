@@ -232,7 +232,7 @@ int vb_create(vb_handle* out, int dims, int nx, int ny, int nz, int nghost, cons
     if (nghost == 0) {
         const int N = nx;
         double* base = nullptr;
-        if ((rc = dev_alloc(h, (void**)&base, sizeof(double) * 7 * 3 * (size_t)N))) {
+        if ((rc = dev_alloc(h, (void**)&base, sizeof(double) * 6 * 3 * (size_t)N))) {
             g_err = h->err;
             delete h;
             return rc;
@@ -244,7 +244,6 @@ int vb_create(vb_handle* out, int dims, int nx, int ny, int nz, int nghost, cons
         h->r1.Uh = base + 9 * N;
         h->r1.PL = base + 12 * N;
         h->r1.PR = base + 15 * N;
-        h->r1.F = base + 18 * N;
     } else {
         size_t pb = (fp32(h) ? sizeof(float) : sizeof(double)) * h->nv * (size_t)h->vs;
         size_t ub = sizeof(double) * h->nv * (size_t)h->vs;
@@ -599,8 +598,10 @@ template <typename R> static int step_nd(vb_handle h, double dt, cudaStream_t s)
         return fail(h, VB_ERR_STATE, "vb_step: FMA-contracted FP64 unit built from another StageParams");
     // the stage's last kernel copies the ghost cells where it has CTAs for them:
     // the split con2prim kernels, the gated learned form's deferred pass, the 1D / 2D box kernel.
-    // The deferred pass, with few threads per SM, takes them up to a million cells: at 512^3
-    // (4.8 M) it took 250 us with them, 28 us without and k_ghost_limit 205 us
+    // The deferred pass, with few threads per SM, takes them up to a million cells, where it is
+    // the faster by a little (a step with it and with k_ghost_limit: 64^3, 0.08 M ghosts,
+    // 206 and 211 us; 200^3, 0.74 M, 3.419 and 3.425 ms; 320^3, 1.9 M, 11.66 and 11.68 ms); at
+    // 512^3, 4.8 M, a stage took 250 us with it against 28 + 205 us
     const bool learned = p.skip_c2p != 0;
     const long long ghosts = h->ncell - (long long)h->n[0] * h->n[1] * h->n[2];
     const bool gated = learned && h->tun.learned_fused != 0 && p.c2p_fp32 && h->defer_idx && ghosts <= (1 << 20);

@@ -118,10 +118,10 @@ template <typename R>
 cudaError_t launch_max_speed(const Grid& g, const R* P, double gamma, double* partial, int max_partial,
                              double* out, cudaStream_t s);
 
-// 1D reference solver (src/1dim/algos.jl:58-315), FP64, one persistent CTA.
+// 1D reference solver (src/1dim/algos.jl:58-315), FP64, one thread-block cluster.
 struct Ref1DState {
     int N;
-    double *P, *Ph, *U, *Uh, *PL, *PR, *F;  // [3][N] each
+    double *P, *Ph, *U, *Uh, *PL, *PR;  // [3][N] each
 };
 cudaError_t launch_ref1d_init(const Ref1DState& st, const double* P_aos, double gamma, cudaStream_t s);
 cudaError_t launch_ref1d_steps(const Ref1DState& st, double gamma, int rec, int n_iter, double tol,
@@ -131,7 +131,7 @@ cudaError_t launch_ref1d_store(const Ref1DState& st, double* P_aos, cudaStream_t
 int max_speed_blocks(const Grid& g);
 
 // FP32-bulk z-pair variant of the 3D stage (vb_stage_zp.cuh, instantiated in
-// vb_stage_f32.cu): WENOZ reconstruction with HLL or HLLC
+// vb_stage_zp_f32.cu): every reconstruction with HLL or HLLC
 inline bool zp_available(int rec, int rs) { return rec >= 0 && rec <= 2 && (rs == 0 || rs == 1); }
 cudaError_t launch_stage_zp(int rec, int rs, const StageParams& p, const StageBufs<float>& b, cudaStream_t s);
 // the y-marching 2D stage of the FP32-bulk form (vb_stage_yp.cuh, p.pairs): writes U, no con2prim

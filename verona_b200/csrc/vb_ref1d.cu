@@ -222,7 +222,6 @@ __global__ void k_ref1d_init(Ref1DState st, const double* __restrict__ Pa, doubl
             st.PR[v * N + i] = p[v];
             st.U[v * N + i] = U[v];
             st.Uh[v * N + i] = U[v];
-            st.F[v * N + i] = 0.0;
         }
     }
 }

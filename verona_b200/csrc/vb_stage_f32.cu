@@ -1,15 +1,12 @@
 // FP32-bulk instantiation: primitive arrays, reconstruction, Riemann fluxes
 // and flux differences in FP32; conserved variables, the RK accumulation and
-// con2prim in FP64. Built with FMA contraction enabled.
+// con2prim in FP64. Built with FMA contraction enabled. The z-pair kernels are in
+// vb_stage_zp_f32.cu, the y-marching ones in vb_stage_yp_f32.cu.
 #include "vb_stage.cuh"
 #include "vb_stage_zm.cuh"
 #include "vb_stage_zp.cuh"
 
 namespace vb {
-cudaError_t launch_stage_zp(int rec, int rs, const StageParams& p, const StageBufs<float>& b, cudaStream_t s) {
-    return dispatch_stage_zp(rec, rs, p, b, s);
-}
-
 // Tensor maps of an FP32 state array. 3D, for the TMA form of the z-pair
 // kernel: dims (x, y, z, variable) with byte strides (4 sy, 4 sz, 4 vs), every
 // one a multiple of 16 (rows are pitched to 4 cells); the box is one plane of

@@ -984,11 +984,5 @@ template <int REC>
 cudaError_t dispatch_stage_zp_rec(int rs, const StageParams& p, const StageBufs<float>& b, cudaStream_t s) {
     return rs == RS_HLLC ? dispatch_stage_zp_rs<REC, RS_HLLC>(p, b, s) : dispatch_stage_zp_rs<REC, RS_HLL>(p, b, s);
 }
-inline cudaError_t dispatch_stage_zp(int rec, int rs, const StageParams& p, const StageBufs<float>& b,
-                                     cudaStream_t s) {
-    if (rec == REC_MINMOD) return dispatch_stage_zp_rec<REC_MINMOD>(rs, p, b, s);
-    if (rec == REC_PPM) return dispatch_stage_zp_rec<REC_PPM>(rs, p, b, s);
-    return dispatch_stage_zp_rec<REC_WENOZ>(rs, p, b, s);
-}
 
 }  // namespace vb

@@ -3,9 +3,10 @@
 // body (stage_tile, vb_stage.cuh) with its loads past L1, the ghosts are filled
 // and floored as in the batch kernel (BatchHalo, batch_ghosts), and the cluster
 // meets once per stage. The kernels of one stage take about as long to launch as
-// to run at this size: N = 1024, MINMOD + HLLC, RK2, 10 steps 377 us in 60 launches,
-// 158 us in one. Longer grids fill the GPU from separate launches and keep
-// them. Built with -fmad=false: the same arithmetic as those kernels, bit for bit.
+// to run at this size: a step of MINMOD + HLLC, RK2 (WENOZ, RK3) takes 15.6 (25.3) us
+// here and 24.6 (35.9) us in separate launches, the same from 256 to 2048 cells.
+// 2048 cells are one tile for each CTA of the widest cluster; longer grids keep the
+// separate launches (24.6 us at 2049, 24.0 at 8192). Built with -fmad=false: the same arithmetic as those kernels, bit for bit.
 #include <algorithm>
 #include <cstring>
 
