@@ -107,7 +107,7 @@ __device__ __forceinline__ void batch_ghosts(const StageParams& q, const BatchPr
 // What a tile's stage body does with the ghosts in its halo (stage_tile,
 // stage_tile_pk): at the first stage of a step every tile that has staged ghost
 // cells puts their filled values in the staged copy, so no tile waits for
-// another's fill. 36 tubes and 12 quadrant problems, two steps, a pass: 4.25 ms,
+// another's fill. 36 tubes and 12 quadrant problems, two steps, a pass: 4.16 ms,
 // against 4.10 ms with the edge tiles filling Pin, which the tiles before a short
 // last one read without an order.
 template <typename R> struct BatchHalo {
@@ -279,6 +279,9 @@ __global__ void __launch_bounds__(batch_nt<R>(), BatchVariants<R>::MINB) k_batch
         const int TXc = pr.dims == 1 ? L1 : TX2, TYc = pr.dims == 1 ? 1 : TY2;
         batch_ghosts<R>(q, pr, b.Pin, b.Pout, e.x, e.y, TXc, TYc, st == 0, s_h.t);
         const BatchHalo<R>& halo = s_h;
+        // no data waits here: without the barrier the compiler forms the tiles' addresses
+        // ahead of it and keeps them in spilled registers (256 problems, a step: 12.28 ms, 11.76 with it)
+        __syncthreads();
         if (pr.dims == 1) {
             if (pr.rec == REC_MINMOD) batch_tile<1, REC_MINMOD, RS, R, L1, 1>(q, b, e.x, 0, smem_raw, halo);
             else if (pr.rec == REC_PPM) batch_tile<1, REC_PPM, RS, R, L1, 1>(q, b, e.x, 0, smem_raw, halo);
