@@ -887,7 +887,7 @@ def config1_measure(rank):
     """Config 1, Marti & Mueller problem 1 on N = 1024 cells to t = 0.4 (1024
     steps, CFL 0.4, gamma 5/3): the reference's own 1D scheme
     (Verona1D.HARM_HLL: MINMOD, HLL, midpoint RK2, no ghosts) on the GPU (one
-    persistent CTA runs every step) and as the oracle's C restatement on one
+    thread-block cluster runs every step) and as the oracle's C restatement on one
     host core; and the configured form (MINMOD + HLLC, RK2, outflow ghosts)
     through the ghosted 1D solver on the GPU and the oracle. zone-updates/s =
     1024 cells x steps / time of the whole run."""
@@ -927,7 +927,7 @@ def config1_measure(rank):
     o.step(dt, dx, steps)
     el_cpu = time.perf_counter() - t0
     out["reference_scheme_hll_rk2"] = {
-        "gpu": {"value": N * steps / el, "seconds": el, "kernel": "k_ref1d_steps (one persistent CTA)"},
+        "gpu": {"value": N * steps / el, "seconds": el, "kernel": "k_ref1d_steps (one thread-block cluster)"},
         "cpu_oracle": {"value": N * steps / el_cpu, "seconds": el_cpu, "cores": 1,
                        "note": "the oracle's C restatement of Verona1D.HARM_HLL (the reference's CPU path)"}}
     xg, P0 = mm1_ghosted(N, g)
