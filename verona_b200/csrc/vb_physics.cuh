@@ -4,9 +4,10 @@
 // the same evaluation order: a + b + c is (a + b) + c, x^2 is x*x, x^3 is
 // x*x*x, min/max propagate NaN, and only the explicit fma() calls of
 // src/2dim/structs.jl:192,205,212 are fused. The FP64 translation unit is
-// compiled with -fmad=false, so for T = double every result is bit-identical
-// to the reference's rounding (IEEE +,-,*,/,sqrt are correctly rounded on
-// sm_100a). The FP32-bulk units use the same code with FP32 constants, except
+// compiled with -fmad=false, so for T = double every result has the
+// reference's rounding (IEEE +,-,*,/,sqrt are correctly rounded on sm_100a; the
+// branch-free divide and square root of vb_fp64.cuh up to 2^-51 ulp from a
+// middle). The FP32-bulk units use the same code with FP32 constants, except
 // for the reconstructions, which have FP32 forms of their own (minmod32,
 // ppm32, wenoz32: the same schemes with sign-bit tests, shared differences
 // and approximate reciprocals).
